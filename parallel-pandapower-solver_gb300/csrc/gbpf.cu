@@ -125,10 +125,10 @@ gbpf::ScratchOffsets gbpf::scratch_offsets(int n, int nv, int nblk, int G, bool 
 struct Shape {
     int NT = 0, G = 0, lg = 0, occ = 1;
     double chain_cap = 1.0;  // the schedule's chain segment cap (make_schedule)
-    DBuf dtaskA, dptrA, dtaskC, dptrC, dheadA, dheadC, dtaskF, dheadF, dptrF;
+    DBuf dtaskA, dptrA, dtaskC, dptrC, dtaskF, dptrF;
     gbpf::DevPlan dp{};
     ~Shape() {
-        for (DBuf* b : {&dtaskA, &dptrA, &dtaskC, &dptrC, &dheadA, &dheadC, &dtaskF, &dheadF, &dptrF})
+        for (DBuf* b : {&dtaskA, &dptrA, &dtaskC, &dptrC, &dtaskF, &dptrF})
             b->release();
     }
 };
@@ -348,59 +348,43 @@ int get_shape(gbpf_solver* s, int NT, int G, Shape** out) {
     sh->occ = std::max(1, occ);
     const gbpf::Plan& p = s->plan;
     gbpf::Schedule sc;
-    gbpf::make_schedule(p, NT / G, sc, s->chain_cap);
+    gbpf::make_schedule(p, NT / 32, 32 / G, sc, s->chain_cap);
     // DIAG tasks carry the "two real pivots" flag (PQ row) in bit 5 of their code
     for (size_t t = 0; t < sc.taskA.size() / 4; ++t) {
-        if ((sc.taskA[4 * t + 1] & 3) == gbpf::TK_DIAG) {
+        if (sc.taskA[4 * t] >= 0 && (sc.taskA[4 * t + 1] & 3) == gbpf::TK_DIAG) {
             const int row = sc.taskA[4 * t + 1] >> gbpf::TASK_ROW_SHIFT;
             if (p.row_pq[row]) sc.taskA[4 * t + 1] |= 32;
         }
     }
-    // the first two pairs of every task inline beside its record: a worker fetches them with
-    // the record, one task ahead, and starts the task's block loads without first waiting for
-    // its pair list
-    auto head_pairs = [&](const std::vector<int>& tasks) {
+    // the first two pairs of every task inline beside its record (8 ints a task): a worker
+    // fetches them with the record, one step ahead, and starts the task's block loads without
+    // first waiting for its pair list
+    auto with_pairs = [&](const std::vector<int>& tasks) {
         const size_t nt = tasks.size() / 4;
-        std::vector<int> head(4 * nt, -1);
+        std::vector<int> rec(8 * nt, -1);
         for (size_t t = 0; t < nt; ++t) {
             const int p0 = tasks[4 * t + 2], p1 = tasks[4 * t + 3];
+            std::copy_n(&tasks[4 * t], 4, &rec[8 * t]);
             for (int k = 0; k < 2 && p0 + k < p1; ++k) {
-                head[4 * t + 2 * k] = p.pairs[2 * (size_t)(p0 + k)];
-                head[4 * t + 2 * k + 1] = p.pairs[2 * (size_t)(p0 + k) + 1];
+                rec[8 * t + 4 + 2 * k] = p.pairs[2 * (size_t)(p0 + k)];
+                rec[8 * t + 5 + 2 * k] = p.pairs[2 * (size_t)(p0 + k) + 1];
             }
         }
-        return head;
+        return rec;
     };
-    CK(upload(sh->dheadA, head_pairs(sc.taskA)));
-    CK(upload(sh->dheadC, head_pairs(sc.taskC)));
-    // substitution-only lists for chord passes: every worker's forward tasks of each level,
-    // the ones it runs inside the full factor-level lists
-    std::vector<int> taskF, ptrF((size_t)p.nlev * sc.W + 1, 0);
-    for (size_t q = 0; q + 1 < sc.ptrA.size(); ++q) {
-        ptrF[q] = (int)(taskF.size() / 4);
-        for (int t = sc.ptrA[q]; t < sc.ptrA[q + 1]; ++t)
-            if ((sc.taskA[4 * (size_t)t + 1] & 3) == gbpf::TK_FWD)
-                for (int k = 0; k < 4; ++k) taskF.push_back(sc.taskA[4 * (size_t)t + k]);
-    }
-    ptrF.back() = (int)(taskF.size() / 4);
-    if (taskF.empty()) taskF.assign(4, 0);  // keeps the upload non-empty for a grid without forward tasks
-    CK(upload(sh->dheadF, head_pairs(taskF)));
-    CK(upload(sh->dtaskF, taskF));
-    CK(upload(sh->dptrF, ptrF));
-    CK(upload(sh->dtaskA, sc.taskA));
+    CK(upload(sh->dtaskF, with_pairs(sc.taskF)));
+    CK(upload(sh->dptrF, sc.ptrF));
+    CK(upload(sh->dtaskA, with_pairs(sc.taskA)));
     CK(upload(sh->dptrA, sc.ptrA));
-    CK(upload(sh->dtaskC, sc.taskC));
+    CK(upload(sh->dtaskC, with_pairs(sc.taskC)));
     CK(upload(sh->dptrC, sc.ptrC));
     sh->dp = s->dp;
-    sh->dp.W = sc.W;
+    sh->dp.W = NT / G;
     sh->dp.taskA = sh->dtaskA.as<int4>();
     sh->dp.ptrA = sh->dptrA.as<int>();
     sh->dp.taskC = sh->dtaskC.as<int4>();
     sh->dp.ptrC = sh->dptrC.as<int>();
-    sh->dp.headA = sh->dheadA.as<int4>();
-    sh->dp.headC = sh->dheadC.as<int4>();
     sh->dp.taskF = sh->dtaskF.as<int4>();
-    sh->dp.headF = sh->dheadF.as<int4>();
     sh->dp.ptrF = sh->dptrF.as<int>();
     *out = sh.get();
     s->shapes.push_back(std::move(sh));
@@ -441,10 +425,7 @@ int upload_plan(gbpf_solver* s) {
     d.ptrA = nullptr;
     d.taskC = nullptr;
     d.ptrC = nullptr;
-    d.headA = nullptr;
-    d.headC = nullptr;
     d.taskF = nullptr;
-    d.headF = nullptr;
     d.ptrF = nullptr;
     d.pairs = s->dpairs.as<int2>();
     d.row_pq = s->drow_pq.as<uint8_t>();

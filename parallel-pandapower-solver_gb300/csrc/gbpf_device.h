@@ -42,15 +42,14 @@ struct DevPlan {
     const int* row_of_bus;   // bus -> block row, -1 for slack
     const int* eval_order;   // the evaluation's bus sweep (reverse Cuthill-McKee)
     const uint8_t* bus_pq;
-    const int4* taskA;
+    // programs of the CTA's warps (plan.h, Schedule), 2 x int4 a task: the task, and its first
+    // two pairs inline (x0, y0, x1, y1; -1 = none)
+    const int4* taskA;       // factor levels with the forward substitution
     const int* ptrA;
-    const int4* taskC;
+    const int4* taskF;       // the forward substitution alone (chord passes)
+    const int* ptrF;
+    const int4* taskC;       // backward substitution
     const int* ptrC;
-    const int4* headA;       // per taskA entry: its first two pairs inline (x0, y0, x1, y1; -1 = none)
-    const int4* headC;       // per taskC entry: likewise
-    const int4* taskF;       // chord passes: the forward tasks of taskA, same levels and workers
-    const int4* headF;
-    const int* ptrF;         // nlev*W + 1
     const int2* pairs;
     const uint8_t* row_pq;   // block row is PQ (two real pivots)
     const int* bus_of_row;

@@ -444,12 +444,15 @@ __device__ __forceinline__ void mm_sub(B4& acc, const B4& a, const B4& b) {
 }
 
 // One batched factorization + substitution pass over the slots flagged in `on` (G <= 32).
-// Worker w = (warp, lane / G) runs its task list of every level for its G slot lanes;
-// the CTA meets at a barrier after each level, forward and backward. Pivot statistics per
-// slot go to smin / smax (as ordered bits). With `solo` a slot index, P is the one-slot
-// schedule and all threads work on that slot. Slots flagged in `chord` keep the factors already
-// in `fac` and run the substitutions only; when every slot of the CTA does (factor_any false),
-// the workers walk the substitution-only lists instead of skipping factor tasks one by one.
+// Every warp runs its program of steps (plan.h, Schedule): worker lane / G of the warp does its
+// task of the step for its G slot lanes; the CTA meets at a barrier after each level, forward
+// and backward. The program is static, so its fetches are taken off the level's critical path:
+// a step's record and first two pairs are fetched one step ahead, across level boundaries, and
+// a level's end one level ahead. Pivot statistics per slot go to smin / smax (as ordered bits).
+// With `solo` a slot index, P is the one-slot schedule and all threads work on that slot. Slots
+// flagged in `chord` keep the factors already in `fac` and run the substitutions only; when
+// every slot of the CTA does (factor_any false), the warps walk the substitution-only programs
+// instead of skipping factor tasks one by one.
 template <typename real, bool TIMED = false>
 __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const double2* R, typename V4<real>::t2* y,
                         const int* on, int lg, unsigned long long* smin, unsigned long long* smax,
@@ -462,8 +465,9 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
     // solo >= 0: one slot left in the CTA; P then carries the one-slot schedule (a worker per
     // thread) and every thread works on that slot
     const int s = solo >= 0 ? solo : lane & ((1 << lg) - 1);
-    const int w = solo >= 0 ? tid : (tid >> 5) * (32 >> lg) + (lane >> lg);
-    const int W = P.W;
+    const int lgw = solo >= 0 ? 5 : 5 - lg;        // workers per warp (log2), and this lane's worker
+    const int wi = solo >= 0 ? lane : lane >> lg;
+    const int warp = tid >> 5;
     const bool act = on[s] != 0;
     const bool factor = !(chord && chord[s]);
     // float passes take each task's first two pairs from its head record (the double pass
@@ -471,37 +475,45 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
     constexpr bool HEAD = sizeof(real) == 4;
     real pmin = sizeof(real) == 4 ? (real)FLT_MAX : (real)DBL_MAX, pmax = 0;
     B4 dinv = z4<B4>();  // the worker's last inverse diagonal block: scales the L column after it
+    int t = 0, t1 = 0;  // the warp's step, the end of the level's steps
+    int4 next = make_int4(-1, 0, 0, 0), nhead = next;
+    auto fetch = [&](const int4* task) {
+        const int4* rec = task + 2 * (((size_t)t << lgw) + wi);
+        next = __ldg(rec);
+        if constexpr (HEAD) nhead = __ldg(rec + 1);
+    };
+    if (act) {
+        const int* ptr = (factor_any ? P.ptrA : P.ptrF) + warp * (P.nlev + 1);
+        t = __ldg(ptr);
+        t1 = __ldg(ptr + 1);
+        fetch(factor_any ? P.taskA : P.taskF);
+    }
     for (int h = 0; h < P.nlev; ++h) {
         if (act) {
-            const int* const PA = factor_any ? P.ptrA : P.ptrF;
-            const int4* const TA = factor_any ? P.taskA : P.taskF;
-            const int4* const HA = factor_any ? P.headA : P.headF;
-            const int t0 = __ldg(&PA[h * W + w]), t1 = __ldg(&PA[h * W + w + 1]);
-            // the next task's record and first two pairs are fetched while the current one
-            // runs, so a task's block loads all go out at once when it starts
-            int4 next = make_int4(0, 0, 0, 0), nhead = make_int4(0, 0, 0, 0);
-            if (t0 < t1) {
-                next = __ldg(&TA[t0]);
-                if constexpr (HEAD) nhead = __ldg(&HA[t0]);
-            }
-            for (int t = t0; t < t1; ++t) {
+            const int t2 = __ldg((factor_any ? P.ptrA : P.ptrF) + warp * (P.nlev + 1) + h + 2);
+            while (t < t1) {
                 const int4 task = next, hd = nhead;
-                if (t + 1 < t1) {
-                    next = __ldg(&TA[t + 1]);
-                    if constexpr (HEAD) nhead = __ldg(&HA[t + 1]);
-                }
+                ++t;
+                fetch(factor_any ? P.taskA : P.taskF);
+                if (task.x < 0) continue;  // no task for this worker in the step
                 const int kind = task.y & 3;
                 const int np = HEAD ? min(task.w - task.z, 2) : 0;  // pairs taken from the head
                 if (kind != 3 && !factor) continue;
                 if (kind == 3) {  // forward substitution of block row task.x
-                    const double2 r = R[((size_t)task.x << lg) + s];
                     real y0, y1;
-                    if constexpr (sizeof(real) == 4) {
-                        y0 = d2f_fast(r.x);
-                        y1 = d2f_fast(r.y);
-                    } else {
+                    if (task.y & 128) {  // its leading pairs are already summed (TASK_CONT)
+                        const B2 r = y[((size_t)task.x << lg) + s];
                         y0 = r.x;
                         y1 = r.y;
+                    } else {
+                        const double2 r = R[((size_t)task.x << lg) + s];
+                        if constexpr (sizeof(real) == 4) {
+                            y0 = d2f_fast(r.x);
+                            y1 = d2f_fast(r.y);
+                        } else {
+                            y0 = r.x;
+                            y1 = r.y;
+                        }
                     }
                     if (np > 0) {
                         const B4 l0 = fac[((size_t)hd.x << lg) + s];
@@ -610,24 +622,25 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
                     fac[((size_t)task.x << lg) + s] = acc;
                 }
             }
+            t1 = t2;
         }
         __syncthreads();
     }
     if constexpr (TIMED) phase_mark(ph, clk, 1);
+    if (act) {
+        const int* ptr = P.ptrC + warp * (P.nblev + 1);
+        t = __ldg(ptr);
+        t1 = __ldg(ptr + 1);
+        fetch(P.taskC);
+    }
     for (int h = 0; h < P.nblev; ++h) {
         if (act) {
-            const int t0 = __ldg(&P.ptrC[h * W + w]), t1 = __ldg(&P.ptrC[h * W + w + 1]);
-            int4 next = make_int4(0, 0, 0, 0), nhead = make_int4(0, 0, 0, 0);
-            if (t0 < t1) {
-                next = __ldg(&P.taskC[t0]);
-                if constexpr (HEAD) nhead = __ldg(&P.headC[t0]);
-            }
-            for (int t = t0; t < t1; ++t) {
+            const int t2 = __ldg(P.ptrC + warp * (P.nblev + 1) + h + 2);
+            while (t < t1) {
                 const int4 task = next, hd = nhead;
-                if (t + 1 < t1) {
-                    next = __ldg(&P.taskC[t + 1]);
-                    if constexpr (HEAD) nhead = __ldg(&P.headC[t + 1]);
-                }
+                ++t;
+                fetch(P.taskC);
+                if (task.x < 0) continue;
                 const int np = HEAD ? min(task.w - task.z, 2) : 0;  // pairs taken from the head
                 const B2 yr = y[((size_t)task.x << lg) + s];
                 const B4 d = fac[((size_t)task.y << lg) + s];
@@ -675,6 +688,7 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
                 o.y = fmadd(d.z, r0, mulr(d.w, r1));
                 y[((size_t)task.x << lg) + s] = o;
             }
+            t1 = t2;
         }
         __syncthreads();
     }

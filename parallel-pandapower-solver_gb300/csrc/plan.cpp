@@ -114,31 +114,34 @@ std::vector<int> rcm_order(int n, const int* Yp, const int* Yj) {
     return order;
 }
 
-// Lay tasks out grouped by (level, worker); `four`: 4 ints per record (else 2). Chains
-// (a diagonal and its L column) go to one worker; a chain heavier than its level's share of a
-// worker (total weight / W) is cut into segments of at most that share (at least one L block
-// each), every segment after the first led by a copy of the diagonal task flagged
-// TASK_NOSTORE (it recomputes the inverse from the Jacobian's diagonal, which the pass
-// leaves in place). Units are dealt longest-first onto the least-loaded worker.
-void layout(const std::vector<Task>& tasks, int nlev, int W, std::vector<int>& out, std::vector<int>& ptr,
-            std::vector<int>* level_work, bool four, const std::vector<int>* key = nullptr, double chain_cap = 1.0) {
+// Lay tasks out as one program per warp: its steps of every level, `wpw` tasks a step (one per
+// worker of the warp, destination -1 where there is none). Chains (a diagonal and its L column) go to
+// one worker; a chain heavier than its level's share of a worker (total weight / workers) is cut
+// into segments of at most that share (at least one L block each), every segment after the first
+// led by a copy of the diagonal task flagged TASK_NOSTORE (it recomputes the inverse from the
+// Jacobian's diagonal, which the pass leaves in place).
+//
+// A warp's workers run in step, so a level's units (chains, segments, single tasks) are first
+// tied into bundles of wpw units alike -- factor and forward units apart, neighbours in weight --
+// and the bundles are dealt to warps heaviest first onto the least-loaded one. Full bundles cost
+// a narrow level its spread over the CTA's warps, but one unit per warp instead (2,000-bus grid,
+// one case: mixed 0.907 ms against 0.887 bundled, double 1.80 against 1.52; 118 buses, one case:
+// 0.493 against 0.414 double) issues every instruction once per unit, and a double-precision one
+// keeps the SM's FP64 pipe for 16 cycles however few of its lanes work.
+void layout(const std::vector<Task>& tasks, int nlev, int nwarps, int wpw, std::vector<int>& out,
+            std::vector<int>& ptr, std::vector<int>* level_work, const std::vector<int>& key, double chain_cap, bool mixed_kinds) {
     std::vector<std::vector<int>> by_level(nlev);
     for (int i = 0; i < (int)tasks.size(); ++i)
         if (tasks[i].head) by_level[tasks[i].level].push_back(i);
-    ptr.assign((size_t)nlev * W + 1, 0);
-    out.clear();
-    std::vector<long long> wts;
-    std::vector<int> who;
-    std::vector<std::vector<int>> units;  // task indices; ~i = a recomputing copy of diagonal task i
-    auto emit = [&](int q) {
-        const Task& t = tasks[q < 0 ? ~q : q];
-        out.push_back(t.dst);
-        out.push_back(q < 0 ? (t.code | TASK_NOSTORE) : t.code);
-        if (four) {
-            out.push_back(t.p0);
-            out.push_back(t.p1);
-        }
-    };
+    const int W = nwarps * wpw;
+    std::vector<long long> wts, bw;
+    std::vector<int> who, idx;
+    std::vector<std::vector<int>> units;    // task indices; ~i = a recomputing copy of diagonal task i
+    std::vector<std::vector<int>> bundles;  // unit indices
+    using Bundle = std::vector<std::vector<int>>;                // its units' task lists
+    std::vector<std::vector<std::vector<Bundle>>> mine(nwarps);  // [warp][level]
+    for (auto& m : mine) m.resize(nlev);
+    auto task_of = [](int q) { return q < 0 ? ~q : q; };
     for (int h = 0; h < nlev; ++h) {
         const auto& ids = by_level[h];
         long long total = 0;
@@ -176,28 +179,68 @@ void layout(const std::vector<Task>& tasks, int nlev, int W, std::vector<int>& o
             }
             wts.push_back(uw);
         }
-        const int mx = deal(wts, W, who);
-        if (level_work) (*level_work)[h] += mx;
-        // within a worker, units in the order of their key (the factor position they work
-        // on): at any moment the workers of a CTA are at similar positions and share the
-        // blocks they read in cache
-        std::vector<int> mine;
-        for (int w = 0; w < W; ++w) {
-            ptr[(size_t)h * W + w] = four ? (int)(out.size() / 4) : (int)(out.size() / 2);
-            mine.clear();
-            for (size_t i = 0; i < units.size(); ++i)
-                if (who[i] == w) mine.push_back((int)i);
-            if (key)
-                std::stable_sort(mine.begin(), mine.end(), [&](int a, int b) {
-                    const int qa = units[a][0] < 0 ? ~units[a][0] : units[a][0];
-                    const int qb = units[b][0] < 0 ? ~units[b][0] : units[b][0];
-                    return (*key)[qa] < (*key)[qb];
-                });
-            for (int i : mine)
-                for (int q : units[i]) emit(q);
+        const int nu = (int)units.size();
+                idx.resize(nu);
+        for (int i = 0; i < nu; ++i) idx[i] = i;
+        auto fwd = [&](int i) { return mixed_kinds && (tasks[task_of(units[i][0])].code & 3) == TK_FWD; };
+        std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
+            return fwd(a) != fwd(b) ? !fwd(a) : wts[a] > wts[b];
+        });
+        bundles.clear();
+        bw.clear();
+        for (int i = 0; i < nu; ++i) {
+            if (bundles.empty() || (int)bundles.back().size() >= wpw || fwd(bundles.back()[0]) != fwd(idx[i])) {
+                bundles.emplace_back();
+                bw.push_back(0);
+            }
+            bundles.back().push_back(idx[i]);
+            bw.back() = std::max(bw.back(), wts[idx[i]]);
         }
+        const int mx = deal(bw, nwarps, who);
+        if (level_work) (*level_work)[h] += mx;
+        for (size_t b = 0; b < bundles.size(); ++b) {
+            auto& dst = mine[who[b]][h];
+            dst.emplace_back();
+            for (int u : bundles[b]) dst.back().push_back(units[u]);
+        }
+        // within a warp, bundles in the order of their key (the factor position they work on):
+        // at any moment the warps of a CTA are at similar positions and share the blocks they
+        // read in cache
+        for (auto& m : mine)
+            std::stable_sort(m[h].begin(), m[h].end(), [&](const auto& a, const auto& b) {
+                return key[task_of(a[0][0])] < key[task_of(b[0][0])];
+            });
     }
-    ptr[(size_t)nlev * W] = four ? (int)(out.size() / 4) : (int)(out.size() / 2);
+    out.clear();
+    ptr.clear();
+    const int null_task[4] = {-1, 0, 0, 0};
+    int steps = 0;
+    for (int u = 0; u < nwarps; ++u) {
+        for (int h = 0; h < nlev; ++h) {
+            ptr.push_back(steps);
+            for (const auto& bundle : mine[u][h]) {
+                size_t len = 0;
+                for (const auto& unit : bundle) len = std::max(len, unit.size());
+                for (size_t k = 0; k < len; ++k, ++steps)
+                    for (int w = 0; w < wpw; ++w) {
+                        if (w >= (int)bundle.size() || k >= bundle[w].size()) {
+                            out.insert(out.end(), null_task, null_task + 4);
+                            continue;
+                        }
+                        const int q = bundle[w][k];
+                        const Task& t = tasks[task_of(q)];
+                        out.push_back(t.dst);
+                        out.push_back(q < 0 ? (t.code | TASK_NOSTORE) : t.code);
+                        out.push_back(t.p0);
+                        out.push_back(t.p1);
+                    }
+            }
+        }
+        ptr.push_back(steps);
+    }
+    // read ahead by the kernel: a step past the last, a range past the last level
+    for (int w = 0; w < wpw; ++w) out.insert(out.end(), null_task, null_task + 4);
+    ptr.push_back(steps);
 }
 
 }  // namespace
@@ -344,7 +387,7 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
     std::vector<int> poff(p.nblk + 1, 0), foff(nv + 1, 0);
     for (int q = 0; q < p.nblk; ++q) poff[q + 1] = poff[q] + pcount[q];
     for (int i = 0; i < nv; ++i) foff[i + 1] = foff[i] + fcount[i];
-    std::vector<int> fpairs(2 * (size_t)poff[p.nblk]), fwd(2 * (size_t)foff[nv]);
+    std::vector<int> fpairs(2 * (size_t)poff[p.nblk]), fwd(2 * (size_t)foff[nv]), fsrc(poff[p.nblk]);
     std::vector<int> pfill(poff.begin(), poff.end() - 1), ffill(foff.begin(), foff.end() - 1);
     for (int s = 0; s < nv; ++s) {
         const int lo = p.Lp[s], hi = p.Lp[s + 1];
@@ -359,6 +402,7 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
                 const int q = pfill[pos(a, b)]++;
                 fpairs[2 * q] = la;
                 fpairs[2 * q + 1] = posU(s, b);
+                fsrc[q] = s;
             }
         }
     }
@@ -367,11 +411,13 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
     const int W = p.W = std::max(1, workers);
     std::vector<Task> A, C;
     p.pairs.clear();
+    p.pair_level.clear();
     auto add_pairs_factor = [&](int q, int& p0, int& p1) {
         p0 = (int)(p.pairs.size() / 2);
         for (int e = poff[q]; e < poff[q + 1]; ++e) {
             p.pairs.push_back(fpairs[2 * e]);
             p.pairs.push_back(fpairs[2 * e + 1]);
+            p.pair_level.push_back(p.height[fsrc[e]]);
         }
         p1 = (int)(p.pairs.size() / 2);
     };
@@ -406,6 +452,7 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
         for (int e = foff[t]; e < foff[t + 1]; ++e) {
             p.pairs.push_back(fwd[2 * e]);
             p.pairs.push_back(fwd[2 * e + 1]);
+            p.pair_level.push_back(p.height[fwd[2 * e + 1]]);
         }
         p1 = (int)(p.pairs.size() / 2);
         p.n_fwd_pairs += p1 - p0;
@@ -415,6 +462,7 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
         for (int x = p.Lp[t]; x < p.Lp[t + 1]; ++x) {
             p.pairs.push_back(posU(t, p.Li[x]));
             p.pairs.push_back(p.Li[x]);
+            p.pair_level.push_back(-1);
         }
         p1 = (int)(p.pairs.size() / 2);
         p.n_bwd_pairs += p1 - p0;
@@ -423,29 +471,104 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
     if (p.pairs.size() / 2 >= (size_t)1 << 31) return "too many pairs";
     p.tasksA = std::move(A);
     p.tasksC = std::move(C);
+    p.warp = std::min(32, std::max(1, W / 16));
+    while (W % p.warp) --p.warp;
     Schedule sc;
-    make_schedule(p, W, sc, chain_cap);
+    make_schedule(p, W / p.warp, p.warp, sc, chain_cap);
     p.taskA = std::move(sc.taskA);
     p.ptrA = std::move(sc.ptrA);
+    p.taskF = std::move(sc.taskF);
+    p.ptrF = std::move(sc.ptrF);
     p.taskC = std::move(sc.taskC);
     p.ptrC = std::move(sc.ptrC);
     p.level_work = std::move(sc.level_work);
     return std::string();
 }
 
-void make_schedule(const Plan& p, int workers, Schedule& out, double chain_cap) {
-    const int W = out.W = std::max(1, workers);
+namespace {
+
+// Dependent memory round trips of a task: its block and first two pairs load together, every
+// two further pairs wait for one more.
+int round_trips(const Task& t) { return 1 + std::max(0, (t.p1 - t.p0 - 1) / 2); }
+
+// The part of long tasks that does not have to wait for its level: a task's pairs are summed in
+// ascending pivot order, and in the upper, narrow levels of the elimination tree most of a
+// block's (or forward row's) pairs come from far below, so that its leading pairs can be summed
+// earlier, where the levels are wide. Level by level from the top, a unit that takes longer than
+// its level's mean load of a worker has its tasks cut: the longest leading run of pairs that
+// is final two levels below becomes a task of its own right above the last of them (a U task
+// into the same block, or a forward task into the same row), and the task itself continues
+// from the stored sum (TASK_CONT: a forward row reads its y). The sums keep their order, so
+// every rounding is the uncut task's. A level's mean is the line because a shorter unit hides
+// behind the rest of its level and a cut costs one more read and write of the block. One case
+// of the 2,000-bus grid: 335 dependent round trips become 159, factorization and forward
+// substitution 0.61 -> 0.44 ms (19,999 buses 2.40 -> 1.66); 730 lanes of it, 4 cases a CTA:
+// 16.4 -> 12.1 ms; 8,760 cases, 32 a CTA: mixed 3.14 -> 2.74 ms, double 7.29 -> 6.80 ms.
+std::vector<Task> cut_long(const Plan& p, std::vector<Task> tasks, int nlev, int workers) {
+    std::vector<std::vector<int>> at(nlev);
+    std::vector<long long> load(nlev, 0);
+    for (int i = 0; i < (int)tasks.size(); ++i) {
+        load[tasks[i].level] += round_trips(tasks[i]);
+        if (tasks[i].head) at[tasks[i].level].push_back(i);
+    }
+    for (int h = nlev - 1; h > 0; --h) {
+        const auto ids = at[h];
+        const long long mean = (load[h] + workers - 1) / workers;
+        for (int id : ids) {
+            long long unit = 0;
+            for (int q = id; q >= 0; q = tasks[q].next) unit += round_trips(tasks[q]);
+            if (unit <= mean) continue;
+            for (int q = id; q >= 0; q = tasks[q].next) {
+                const Task t = tasks[q];
+                int c = 0, top = -1;
+                for (int e = t.p0; e < t.p1 && p.pair_level[e] <= h - 2; ++e, ++c) top = std::max(top, p.pair_level[e]);
+                Task rest = t;
+                rest.p0 += c;
+                if (c == 0 || round_trips(rest) >= round_trips(t)) continue;
+                const bool fwd = (t.code & 3) == TK_FWD;
+                Task lead = t;
+                lead.level = top + 1;
+                lead.p1 = rest.p0;
+                lead.code = fwd ? t.code : TK_U | (t.code & TASK_FILL);
+                lead.next = -1;
+                lead.head = true;
+                lead.w = (fwd ? 4LL : 8LL) * c + (fwd ? 4 : 8);
+                rest.code = fwd ? t.code | TASK_CONT : t.code & ~TASK_FILL;
+                rest.w = t.w - (fwd ? 4LL : 8LL) * c;
+                load[h] += round_trips(rest) - round_trips(t);
+                load[lead.level] += round_trips(lead);
+                tasks[q] = rest;
+                at[lead.level].push_back((int)tasks.size());
+                tasks.push_back(lead);
+            }
+        }
+    }
+    return tasks;
+}
+
+}  // namespace
+
+void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double chain_cap) {
+    out.nwarps = std::max(1, nwarps);
+    out.wpw = std::max(1, wpw);
     out.level_work.assign(std::max(p.nlev, p.nblev), 0);
     // factor-level key: the task's destination block (a forward row: its diagonal block)
-    std::vector<int> keyA(p.tasksA.size());
-    for (size_t i = 0; i < p.tasksA.size(); ++i) {
-        const Task& t = p.tasksA[i];
-        keyA[i] = (t.code & 3) == TK_FWD ? p.base[t.dst] : t.dst;
-    }
-    layout(p.tasksA, p.nlev, W, out.taskA, out.ptrA, &out.level_work, true, &keyA, chain_cap);
-    std::vector<int> keyC(p.tasksC.size());
-    for (size_t i = 0; i < p.tasksC.size(); ++i) keyC[i] = p.tasksC[i].dst;
-    layout(p.tasksC, p.nblev, W, out.taskC, out.ptrC, nullptr, true, &keyC, chain_cap);
+    auto keys = [&](const std::vector<Task>& tasks, bool rows) {
+        std::vector<int> key(tasks.size());
+        for (size_t i = 0; i < tasks.size(); ++i)
+            key[i] = !rows && (tasks[i].code & 3) == TK_FWD ? p.base[tasks[i].dst] : tasks[i].dst;
+        return key;
+    };
+    std::vector<Task> fwd;  // the substitution-only passes' lists, dealt on their own
+    for (const Task& t : p.tasksA)
+        if ((t.code & 3) == TK_FWD) fwd.push_back(t);
+    const int workers = out.nwarps * out.wpw;
+    const std::vector<Task> A = cut_long(p, p.tasksA, p.nlev, workers);
+    fwd = cut_long(p, fwd, p.nlev, workers);
+    layout(A, p.nlev, out.nwarps, out.wpw, out.taskA, out.ptrA, &out.level_work, keys(A, false), chain_cap, true);
+    layout(fwd, p.nlev, out.nwarps, out.wpw, out.taskF, out.ptrF, nullptr, keys(fwd, false), chain_cap, false);
+    layout(p.tasksC, p.nblev, out.nwarps, out.wpw, out.taskC, out.ptrC, nullptr, keys(p.tasksC, true), chain_cap,
+           false);
 }
 
 // ----------------------------------------------------------------------------- host replica
@@ -511,6 +634,14 @@ void host_eval(const Plan& p, const int* Yp, const int* Yj, const double* Yx, co
     }
 }
 
+// Steps of worker w's warp in level h of a schedule's range list.
+static inline int first_step(const Plan& p, const std::vector<int>& ptr, int nlev, int h, int w) {
+    return ptr[(size_t)(w / p.warp) * (nlev + 1) + h];
+}
+static inline int last_step(const Plan& p, const std::vector<int>& ptr, int nlev, int h, int w) {
+    return ptr[(size_t)(w / p.warp) * (nlev + 1) + h + 1];
+}
+
 static inline void mm_sub(double* acc, const double* a, const double* b) {
     acc[0] -= a[0] * b[0] + a[1] * b[2];
     acc[1] -= a[0] * b[1] + a[1] * b[3];
@@ -521,14 +652,13 @@ static inline void mm_sub(double* acc, const double* a, const double* b) {
 bool host_factor(const Plan& p, double* blk, double* pmin, double* pmax) {
     double mn = INFINITY, mx = 0.0;
     bool ok = true;
-    const int W = p.W;
     for (int h = 0; h < p.nlev; ++h) {
-        for (int w = 0; w < W; ++w) {
+        for (int w = 0; w < p.W; ++w) {
             double dinv[4] = {0, 0, 0, 0};  // the worker's last inverse diagonal block
-            for (int t = p.ptrA[(size_t)h * W + w]; t < p.ptrA[(size_t)h * W + w + 1]; ++t) {
-                const int* T = &p.taskA[4 * (size_t)t];
+            for (int t = first_step(p, p.ptrA, p.nlev, h, w); t < last_step(p, p.ptrA, p.nlev, h, w); ++t) {
+                const int* T = &p.taskA[4 * ((size_t)t * p.warp + w % p.warp)];
                 const int kind = T[1] & 3;
-                if (kind == TK_FWD) continue;
+                if (kind == TK_FWD || T[0] < 0) continue;
                 double acc[4] = {0, 0, 0, 0};
                 if (!(T[1] & TASK_FILL))
                     for (int e = 0; e < 4; ++e) acc[e] = blk[4 * (size_t)T[0] + e];
@@ -609,18 +739,23 @@ std::string schedule_selftest(const Plan& p, double* blk, const double* R, doubl
     for (int h = 0; h < p.nlev; ++h) {
         // structural: writes of the factor level
         for (int w = 0; w < W; ++w)
-            for (int t = p.ptrA[(size_t)h * W + w]; t < p.ptrA[(size_t)h * W + w + 1]; ++t) {
-                const int* T = &p.taskA[4 * (size_t)t];
-                if ((T[1] & 3) == TK_FWD)
+            for (int t = first_step(p, p.ptrA, p.nlev, h, w); t < last_step(p, p.ptrA, p.nlev, h, w); ++t) {
+                const int* T = &p.taskA[4 * ((size_t)t * p.warp + w % p.warp)];
+                if (T[0] < 0) continue;
+                if (((T[1] & 3) == TK_FWD ? ystamp[T[0]] : wstamp[T[0]]) == h && !(T[1] & TASK_NOSTORE))
+                    return "level " + std::to_string(h) + ": a block or row is written twice in its level";
+                if ((T[1] & 3) == TK_FWD) {
+                    if ((T[1] & TASK_CONT) && ystamp[T[0]] < 0) return "a forward row goes on from no sum";
                     ystamp[T[0]] = h;
-                else if ((T[1] & 3) == TK_DIAG) {  // writes its inverse; the Jacobian's block stays
+                } else if ((T[1] & 3) == TK_DIAG) {  // writes its inverse; the Jacobian's block stays
                     if (!(T[1] & TASK_NOSTORE)) wstamp[(size_t)p.nblk + (T[1] >> TASK_ROW_SHIFT)] = h;
                 } else
                     wstamp[T[0]] = h;
             }
         for (int w = 0; w < W; ++w)
-            for (int t = p.ptrA[(size_t)h * W + w]; t < p.ptrA[(size_t)h * W + w + 1]; ++t) {
-                const int* T = &p.taskA[4 * (size_t)t];
+            for (int t = first_step(p, p.ptrA, p.nlev, h, w); t < last_step(p, p.ptrA, p.nlev, h, w); ++t) {
+                const int* T = &p.taskA[4 * ((size_t)t * p.warp + w % p.warp)];
+                if (T[0] < 0) continue;
                 const bool fwd = (T[1] & 3) == TK_FWD;
                 if ((T[1] & 3) == TK_DIAG && wstamp[T[0]] == h)
                     return "level " + std::to_string(h) + ": a diagonal block is rewritten in its level";
@@ -635,11 +770,13 @@ std::string schedule_selftest(const Plan& p, double* blk, const double* R, doubl
         for (int w = W - 1; w >= 0; --w) {
             double dinv[4] = {0, 0, 0, 0};
             int dinv_level = -1;
-            for (int t = p.ptrA[(size_t)h * W + w]; t < p.ptrA[(size_t)h * W + w + 1]; ++t) {
-                const int* T = &p.taskA[4 * (size_t)t];
+            for (int t = first_step(p, p.ptrA, p.nlev, h, w); t < last_step(p, p.ptrA, p.nlev, h, w); ++t) {
+                const int* T = &p.taskA[4 * ((size_t)t * p.warp + w % p.warp)];
+                if (T[0] < 0) continue;
                 const int kind = T[1] & 3;
                 if (kind == TK_FWD) {
-                    double y0 = R[2 * T[0]], y1 = R[2 * T[0] + 1];
+                    const double* from = (T[1] & TASK_CONT) ? y : R;
+                    double y0 = from[2 * T[0]], y1 = from[2 * T[0] + 1];
                     for (int q = T[2]; q < T[3]; ++q) {
                         const double* l = blk + 4 * (size_t)p.pairs[2 * q];
                         const int srow = p.pairs[2 * q + 1];
@@ -685,13 +822,37 @@ std::string schedule_selftest(const Plan& p, double* blk, const double* R, doubl
             }
         }
     }
+    // the substitution-only programs on the finished factors: the same y, bit for bit
+    std::vector<double> y2(2 * (size_t)std::max(p.nv, 1), 0.0);
+    for (int h = 0; h < p.nlev; ++h)
+        for (int w = W - 1; w >= 0; --w)
+            for (int t = first_step(p, p.ptrF, p.nlev, h, w); t < last_step(p, p.ptrF, p.nlev, h, w); ++t) {
+                const int* T = &p.taskF[4 * ((size_t)t * p.warp + w % p.warp)];
+                if (T[0] < 0) continue;
+                const double* from = (T[1] & TASK_CONT) ? y2.data() : R;
+                double y0 = from[2 * T[0]], y1 = from[2 * T[0] + 1];
+                for (int q = T[2]; q < T[3]; ++q) {
+                    const double* l = blk + 4 * (size_t)p.pairs[2 * q];
+                    const int srow = p.pairs[2 * q + 1];
+                    y0 -= l[0] * y2[2 * srow] + l[1] * y2[2 * srow + 1];
+                    y1 -= l[2] * y2[2 * srow] + l[3] * y2[2 * srow + 1];
+                }
+                y2[2 * T[0]] = y0;
+                y2[2 * T[0] + 1] = y1;
+            }
+    for (int k = 0; k < 2 * p.nv; ++k)
+        if (y2[k] != y[k]) return "the substitution-only lists give another forward solution";
     std::vector<int> bst(std::max(p.nv, 1), -1);
     for (int h = 0; h < p.nblev; ++h) {
         for (int w = 0; w < W; ++w)
-            for (int t = p.ptrC[(size_t)h * W + w]; t < p.ptrC[(size_t)h * W + w + 1]; ++t) bst[p.taskC[4 * (size_t)t]] = h;
+            for (int t = first_step(p, p.ptrC, p.nblev, h, w); t < last_step(p, p.ptrC, p.nblev, h, w); ++t) {
+                const int* T = &p.taskC[4 * ((size_t)t * p.warp + w % p.warp)];
+                if (T[0] >= 0) bst[T[0]] = h;
+            }
         for (int w = W - 1; w >= 0; --w)
-            for (int t = p.ptrC[(size_t)h * W + w]; t < p.ptrC[(size_t)h * W + w + 1]; ++t) {
-                const int* T = &p.taskC[4 * (size_t)t];
+            for (int t = first_step(p, p.ptrC, p.nblev, h, w); t < last_step(p, p.ptrC, p.nblev, h, w); ++t) {
+                const int* T = &p.taskC[4 * ((size_t)t * p.warp + w % p.warp)];
+                if (T[0] < 0) continue;
                 double r0 = y[2 * T[0]], r1 = y[2 * T[0] + 1];
                 for (int q = T[2]; q < T[3]; ++q) {
                     const double* u = blk + 4 * (size_t)p.pairs[2 * q];

@@ -35,6 +35,7 @@ constexpr int TASK_SCALE = 1 << 3;  // L block: multiply by the inverse diagonal
 constexpr int TASK_FILL = 1 << 4;   // block not in the Jacobian: accumulate from zero
 // (bit 5: the diagonal block has two real pivots -- a PQ row; set when a schedule is uploaded)
 constexpr int TASK_NOSTORE = 1 << 6;  // diagonal recomputed for a chain segment: keep the inverse in registers
+constexpr int TASK_CONT = 1 << 7;     // forward row whose leading pairs are already summed in its y
 constexpr int TASK_ROW_SHIFT = 8;     // diagonal tasks: block row in code >> 8 (inverse at block nblk + row)
 
 // One unit of factorization work before it is dealt to a worker: its level, destination
@@ -46,11 +47,16 @@ struct PlanTask {
     bool head = true;  // first task of a chain (or a task on its own)
 };
 
-// The worker-dependent part of a plan: the level tasks dealt to W workers.
+// The worker-dependent part of a plan: the level tasks dealt to `nwarps` warps of `wpw` workers
+// each. A warp's program is its steps of level 0, 1, ...; step s holds the tasks of its workers
+// at [s * wpw, (s + 1) * wpw) (4 ints each, destination -1: none), and warp u's steps of level h
+// are [ptr[u * (levels + 1) + h], ptr[u * (levels + 1) + h + 1]). One spare step and one spare
+// pointer at the end are read ahead by the kernel.
 struct Schedule {
-    int W = 0;
-    std::vector<int> taskA, ptrA;   // entry tasks (4 ints) and per-(level, worker) ranges
-    std::vector<int> taskC, ptrC;   // backward substitution tasks (4 ints)
+    int nwarps = 0, wpw = 0;
+    std::vector<int> taskA, ptrA;   // factor levels with the forward substitution
+    std::vector<int> taskF, ptrF;   // the forward substitution alone (chord passes)
+    std::vector<int> taskC, ptrC;   // backward substitution
     std::vector<int> level_work;    // per level: max worker load
 };
 
@@ -76,13 +82,15 @@ struct Plan {
     std::vector<int> posmap;        // Ybus nnz -> block position, -1 if a slack is involved
     std::vector<int> ydiag;         // bus -> CSR index of its diagonal, -1 if none
     // schedule for W workers
-    int W = 0;
+    int W = 0, warp = 1;            // workers, workers per warp
     int nlev = 0, nblev = 0;
-    std::vector<int> taskA;         // 4 ints per task: dst, kind|flags, p0, p1
-    std::vector<int> ptrA;          // nlev*W + 1
+    std::vector<int> taskA;         // 4 ints per task: dst, kind|flags, p0, p1 (see Schedule)
+    std::vector<int> ptrA;
+    std::vector<int> taskF, ptrF;   // forward rows alone
     std::vector<int> taskC;         // backward: 4 ints: row, inverse-diagonal block, p0, p1
-    std::vector<int> ptrC;          // nblev*W + 1
+    std::vector<int> ptrC;
     std::vector<int> pairs;         // 2 ints per pair
+    std::vector<int> pair_level;    // level that makes a factor / forward pair's operands final
     // undealt tasks (factor levels, backward), kept so other worker counts can be scheduled
     std::vector<PlanTask> tasksA, tasksC;
     // statistics
@@ -97,11 +105,11 @@ struct Plan {
 std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, const int* pv, int npv,
                        const int* pq, int npq, int workers, double chain_cap = 1.0);
 
-// Deal the plan's tasks to `workers` workers (longest first onto the least-loaded one); a
-// level's diagonal-and-L chain heavier than chain_cap x the level's mean work per worker is
-// cut into segments on different workers, each later one recomputing the diagonal inverse
-// (0: chains are never cut).
-void make_schedule(const Plan& p, int workers, Schedule& out, double chain_cap = 1.0);
+// Deal the plan's tasks to `nwarps` warps of `wpw` workers (longest first onto the least-loaded
+// warp); a level's diagonal-and-L chain heavier than chain_cap x the level's mean work per
+// worker is cut into segments on different workers, each later one recomputing the diagonal
+// inverse (0: chains are never cut).
+void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double chain_cap = 1.0);
 
 // Host replica of the device algorithm (double precision): Jacobian blocks at (Vm, Va)
 // written to `blocks` (nblk*4, zero where not in the Jacobian) and residual R (nv*2).
