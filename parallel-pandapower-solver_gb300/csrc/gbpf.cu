@@ -170,7 +170,7 @@ struct gbpf_solver {
     std::mutex shapes_mu;  // launches of several groups on this topology may look up shapes at once
     std::vector<std::unique_ptr<ExecSlot>> slots;  // asynchronous calls (gbpf_solve_lanes_async)
     // topology on the device
-    DBuf dYp, dYj, dY, dY32, dposmap, drow_of_bus, dbus_pq, dpairs, drow_pq, dbus_of_row, ddpos, deval_order;
+    DBuf dYp, dYj, dY, dY32, dposmap, drow_of_bus, dbus_pq, dpairs, drow_pq, dbus_of_row, ddpos, drows, drows_by_len;
     gbpf::DevPlan dp{};  // topology part (schedule fields filled per shape)
     // scratch: one region per CTA (grow-only)
     DBuf scr;
@@ -193,7 +193,7 @@ struct gbpf_solver {
             if (sl->stream) cudaStreamSynchronize(sl->stream);
         slots.clear();
         shapes.clear();
-        for (DBuf* b : {&dYp, &dYj, &dY, &dY32, &dposmap, &drow_of_bus, &dbus_pq, &dpairs, &drow_pq, &dbus_of_row, &deval_order,
+        for (DBuf* b : {&dYp, &dYj, &dY, &dY32, &dposmap, &drow_of_bus, &dbus_pq, &dpairs, &drow_pq, &dbus_of_row, &drows, &drows_by_len,
                         &ddpos, &scr, &bS, &bV0, &bV, &bit, &bcv, &bctl, &blane, &bstp, &bstk, &bstv, &bYd, &bpin,
                         &btab, &bjobs, &bmis, &iin, &iscr, &ibest, &iout, &dbr_f, &dbr_t, &dbr_live, &dbr_pos, &dbr_val,
                         &dslack, &dprio, &dg_ptr, &dg_src, &dshunt})
@@ -395,9 +395,21 @@ int upload_plan(gbpf_solver* s) {
     const gbpf::Plan& p = s->plan;
     CK(upload(s->dYp, s->Yp));
     CK(upload(s->dYj, s->Yj));
-    CK(upload(s->dposmap, p.posmap));
+    std::vector<int> posmap(2 * (size_t)p.nnzY);
+    for (int k = 0; k < p.nnzY; ++k) {
+        posmap[2 * (size_t)k] = p.posmap[k];
+        posmap[2 * (size_t)k + 1] = p.bus_pq[s->Yj[k]];
+    }
+    CK(upload(s->dposmap, posmap));
     CK(upload(s->drow_of_bus, p.row_of_bus));
-    CK(upload(s->deval_order, p.eval_order));
+    std::vector<int4> rows;
+    for (int bus : p.eval_order)
+        if (p.row_of_bus[bus] >= 0)
+            rows.push_back(make_int4(bus, p.row_of_bus[bus], s->Yp[bus],
+                                     (s->Yp[bus + 1] - s->Yp[bus]) << 1 | (p.bus_pq[bus] ? 1 : 0)));
+    CK(upload(s->drows, rows));
+    std::stable_sort(rows.begin(), rows.end(), [](const int4& a, const int4& b) { return (a.w >> 1) > (b.w >> 1); });
+    CK(upload(s->drows_by_len, rows));
     CK(upload(s->dbus_pq, p.bus_pq));
     CK(upload(s->dpairs, p.pairs));
     CK(upload(s->drow_pq, p.row_pq));
@@ -417,9 +429,10 @@ int upload_plan(gbpf_solver* s) {
     d.Yj = s->dYj.as<int>();
     d.Y = s->dY.as<double2>();
     d.Y32 = s->dY32.as<float2>();
-    d.posmap = s->dposmap.as<int>();
+    d.posmap = s->dposmap.as<int2>();
     d.row_of_bus = s->drow_of_bus.as<int>();
-    d.eval_order = s->deval_order.as<int>();
+    d.rows = s->drows.as<int4>();
+    d.rows_by_len = s->drows_by_len.as<int4>();
     d.bus_pq = s->dbus_pq.as<uint8_t>();
     d.taskA = nullptr;
     d.ptrA = nullptr;

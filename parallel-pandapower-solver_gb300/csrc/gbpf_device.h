@@ -38,9 +38,12 @@ struct DevPlan {
     const int* Yj;
     const double2* Y;        // base Ybus values (G + jB)
     const float2* Y32;       // float copy
-    const int* posmap;       // Ybus nnz -> block, -1
+    const int2* posmap;      // Ybus nnz -> block (-1: a slack's), whether its column is a PQ bus
     const int* row_of_bus;   // bus -> block row, -1 for slack
-    const int* eval_order;   // the evaluation's bus sweep (reverse Cuthill-McKee)
+    // the evaluation's sweep over the variable buses, (bus, block row, first nonzero, nonzeros << 1
+    // | PQ) each: in reverse Cuthill-McKee order, and the same sorted by nonzeros (most first)
+    const int4* rows;
+    const int4* rows_by_len;
     const uint8_t* bus_pq;
     // programs of the CTA's warps (plan.h, Schedule), 2 x int4 a task: the task, and its first
     // two pairs inline (x0, y0, x1, y1; -1 = none)

@@ -195,8 +195,11 @@ __device__ __forceinline__ unsigned row_stamp_mask(const EvalCtx& c, int k0, int
     return mask;
 }
 
-__device__ __forceinline__ double2 ybus_val(const EvalCtx& c, int k, unsigned mask) {
-    double2 y = c.ymode == 2 ? c.Yd[(size_t)k * c.sYd + c.ncase] : __ldg(&c.P->Y[k]);
+__device__ __forceinline__ double2 ybus_load(const EvalCtx& c, int k) {
+    return c.ymode == 2 ? c.Yd[(size_t)k * c.sYd + c.ncase] : __ldg(&c.P->Y[k]);
+}
+
+__device__ __forceinline__ double2 less_stamps(const EvalCtx& c, double2 y, int k, unsigned mask) {
     if (mask) {
         for (int e = 0; e < c.nst; ++e)
             if (((mask >> e) & 1u) && c.stk[e] == k) {
@@ -214,10 +217,14 @@ __device__ __forceinline__ void put_block(float4* fac, size_t at, double a, doub
     fac[at] = make_float4((float)a, (float)b, (float)c, (float)d);
 }
 
+// A row's record (DevPlan::rows): bus, block row, first nonzero, nonzeros << 1 | PQ.
 template <int JM, typename FacT>
-__device__ unsigned long long eval_row(const EvalCtx& c, int i, int s, int row, bool pinned, bool pq_i, double2 Ssp,
-                                       FacT* fac, double2* R, bool write_r) {
+__device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool pinned, double2 Ssp, FacT* fac,
+                                       double2* R, bool write_r) {
     const DevPlan& P = *c.P;
+    const int i = rec.x, row = rec.y;
+    const int k0 = rec.z, k1 = rec.z + (rec.w >> 1);
+    const bool pq_i = rec.w & 1;
     const size_t si = ((size_t)i << c.lg) + s;
     const double2 ei = c.Et[si];
     // float copy of the evaluation point for the float Jacobian: (e, f) truncated from the
@@ -226,20 +233,28 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int i, int s, int row, 
     if (JM == 2) vi32 = make_float4(d2f_trunc(ei.x), d2f_trunc(ei.y), pq_i ? c.iv32[si] : 0.f, 0.f);
     double Ir = 0.0, Ii = 0.0, gii = 0.0, bii = 0.0;
     float gii32 = 0.f, bii32 = 0.f;
-    const int k0 = __ldg(&P.Yp[i]), k1 = __ldg(&P.Yp[i + 1]);
     const unsigned mask = row_stamp_mask(c, k0, k1);
-    // the next nonzero's column and phasor are loaded while this one is worked on (the stores
-    // of the Jacobian blocks would otherwise keep them from being issued early)
-    int jn = k0 < k1 ? __ldg(&P.Yj[k0]) : 0;
-    double2 en = k0 < k1 ? c.Et[((size_t)jn << c.lg) + s] : make_double2(0.0, 0.0);
+    // the next nonzero's phasor and admittance and the column after it are loaded while this one
+    // is worked on (the stores of the Jacobian blocks would otherwise keep them from being
+    // issued early, and the phasor would wait for its column)
+    int jn = 0, jn2 = 0;
+    double2 en = make_double2(0.0, 0.0), yn = en;
+    if (k0 < k1) {
+        jn = __ldg(&P.Yj[k0]);
+        yn = ybus_load(c, k0);
+        jn2 = __ldg(&P.Yj[min(k0 + 1, k1 - 1)]);
+        en = c.Et[((size_t)jn << c.lg) + s];
+    }
     for (int k = k0; k < k1; ++k) {
         const int j = jn;
         const double2 ej = en;
+        const double2 y = less_stamps(c, yn, k, mask);
         if (k + 1 < k1) {
-            jn = __ldg(&P.Yj[k + 1]);
+            jn = jn2;
             en = c.Et[((size_t)jn << c.lg) + s];
+            yn = ybus_load(c, k + 1);
+            jn2 = __ldg(&P.Yj[min(k + 2, k1 - 1)]);
         }
-        const double2 y = ybus_val(c, k, mask);
         const size_t sj = ((size_t)j << c.lg) + s;
         Ir = fma(y.x, ej.x, Ir);
         Ir = fma(-y.y, ej.y, Ir);
@@ -261,9 +276,10 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int i, int s, int row, 
             continue;
         }
         if (JM == 0) continue;
-        const int q = __ldg(&P.posmap[k]);
+        const int2 qj = __ldg(&P.posmap[k]);
+        const int q = qj.x;
         if (q < 0) continue;
-        const bool pq_j = __ldg(&P.bus_pq[j]) != 0;
+        const bool pq_j = qj.y != 0;
         const size_t at = ((size_t)q << c.lg) + s;
         if (pinned) {
             put_block(fac, at, 0.0, 0.0, 0.0, 0.0);
@@ -708,6 +724,13 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
     if constexpr (TIMED) phase_mark(ph, clk, 2);
 }
 
+// *at = max(*at, v) in shared memory. The value only rises, so a v not above what is read needs
+// no atomic (which for 64 bits is a compare-and-swap loop, and one round of it per lane of the
+// slot where a warp holds several rows).
+__device__ __forceinline__ void raise_max(unsigned long long* at, unsigned long long v) {
+    if (v > *(volatile unsigned long long*)at) atomicMax(at, v);
+}
+
 __device__ __forceinline__ bool pivots_ok(unsigned long long bmin, unsigned long long bmax, double rc) {
     if (bmax >= 0x7ff0000000000000ULL) return false;  // NaN / Inf pivot
     const double mn = bitsd(bmin), mx = bitsd(bmax);
@@ -816,6 +839,9 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
     // s_first: the case started from the shared start and its first step uses the shared
     // factors; s_nofac: this step solves with factors it does not compute (chord or first)
     __shared__ int s_first[MAX_SLOTS], s_nofac[MAX_SLOTS];
+    // slots with a point to form and evaluate in this pass, and whether the per-bus phases deal
+    // their threads to those slots only (see `lanes_of`)
+    __shared__ int s_act[MAX_SLOTS], s_nact;
     __shared__ int s_share;  // the launch's shared start is usable (its factorization passed)
     __shared__ int s_stk[MAX_SLOTS][MAX_STAMPS];
     __shared__ double2 s_stv[MAX_SLOTS][MAX_STAMPS];
@@ -1066,7 +1092,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                     const double rq = P.bus_pq[bus] != 0 ? Ssp.y + r0.y : 0.0;
                     R[((size_t)row << lg) + s] = make_double2(rp, rq);
                     const unsigned long long a = abs_bits(rp), b = abs_bits(rq);
-                    atomicMax(&s_res[s], b > a ? b : a);
+                    raise_max(&s_res[s], b > a ? b : a);
                 }
             }
         }
@@ -1102,14 +1128,12 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         // Jacobian at the same point first (the values that evaluation would have written)
         const int anylazy = __syncthreads_or(tid < G && s_on32[tid] && !s_nofac[tid] && s_nojac[tid]);
         if (anylazy) {
-            for (int idx = tid; idx < nG; idx += NT) {
+            for (int idx = tid; idx < P.nv << lg; idx += NT) {
                 const int s = idx & (G - 1);
                 if (!(s_on32[s] && !s_nofac[s] && s_nojac[s])) continue;
-                const int bus = idx >> lg;
-                const int row = P.row_of_bus[bus];
-                if (row < 0) continue;
+                const int4 rec = __ldg(&P.rows[idx >> lg]);
                 EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, s_case[s], s_nst[s], s_stk[s], s_stv[s]};
-                eval_row<2>(ec, bus, s, row, spin[idx] != 0, P.bus_pq[bus] != 0, make_double2(0.0, 0.0),
+                eval_row<2>(ec, rec, s, spin[((size_t)rec.x << lg) + s] != 0, make_double2(0.0, 0.0),
                             s_fb[s] ? fac32 : fac32b, R, false);
             }
             __syncthreads();
@@ -1156,15 +1180,12 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                 if (s_reeval[s]) Ei[idx] = recip_nr((s_tb[s] ? Vb1 : Vb0)[idx].x);
             }
             __syncthreads();
-            for (int idx = tid; idx < nG; idx += NT) {
+            for (int idx = tid; idx < P.nv << lg; idx += NT) {
                 const int s = idx & (G - 1);
                 if (!s_reeval[s]) continue;
-                const int bus = idx >> lg;
-                const int row = P.row_of_bus[bus];
-                if (row < 0) continue;
+                const int4 rec = __ldg(&P.rows[idx >> lg]);
                 EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, s_case[s], s_nst[s], s_stk[s], s_stv[s]};
-                eval_row<1>(ec, bus, s, row, spin[idx] != 0, P.bus_pq[bus] != 0, make_double2(0.0, 0.0), fac64, R,
-                            false);
+                eval_row<1>(ec, rec, s, spin[((size_t)rec.x << lg) + s] != 0, make_double2(0.0, 0.0), fac64, R, false);
             }
             __syncthreads();
             if (tid < G && s_reeval[tid]) s_jprec[tid] = 0;
@@ -1196,19 +1217,50 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                 }
             }
         }
-        if (tid < G && (s_on32[tid] || s_on64[tid])) {
-            s_yprec[tid] = s_on64[tid] ? 0 : 1;
-            s_first[tid] = 0;
+        if (tid < 32) {
+            bool live = false;
+            if (tid < G) {
+                if (s_on32[tid] || s_on64[tid]) {
+                    s_yprec[tid] = s_on64[tid] ? 0 : 1;
+                    s_first[tid] = 0;
+                }
+                const int st = s_st[tid];
+                live = st == SL_FRESH || st == SL_ACTIVE || st == SL_NEEDJ || st == SL_BACKTRACK;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, live);
+            if (live) s_act[__popc(m & ((1u << tid) - 1u))] = tid;
+            if (tid == 0) s_nact = __popc(m);
         }
         __syncthreads();
+        // Threads of the per-bus phases: a thread's buses (or rows) k = first, + stride, ... all
+        // belong to one slot. Where at most three quarters of a small CTA's slots take part,
+        // threads are dealt to those slots only: a warp's double-precision instruction holds its
+        // FP64 pipe for 64 cycles whatever its idle lanes. 730 warm-start lanes of the 2,000-bus
+        // grid (4 slots a CTA, 2.4 of them busy): evaluation 10.6 -> 9.2 ms mixed, 17.7 -> 13.0
+        // ms double, with the rows by length below. From 16 slots on a warp keeps one or two
+        // buses for its lanes, with few record loads, instead of straddling more (3,001 cases, 16
+        // slots, 10 busy: evaluation 1.93 ms mixed, 2.09 dealt; N-1 sweeps equal either way).
+        auto deal = [&](int& slot, int& first, int& stride) {
+            const int na = s_nact;
+            if (4 * na <= 3 * G && G < 16) {
+                const int per = NT / max(na, 1);
+                slot = tid < per * na ? s_act[tid % max(na, 1)] : -1;
+                first = tid / max(na, 1);
+                stride = per;
+            } else {
+                slot = tid & (G - 1);
+                first = tid >> lg;
+                stride = NT >> lg;
+            }
+        };
 
         // ---------------------------------------------------------------- step
-        // A thread's elements idx = tid + k NT all belong to slot tid & (G - 1) (NT is a
-        // multiple of G) -- or all to the solo slot -- so the slot's state is read once and the
-        // next element's committed point and step are loaded while the current one is worked on.
+        // The slot's state is read once, and the next element's committed point and step are
+        // loaded while the current one is worked on.
         {
-            const int s = solo >= 0 ? solo : tid & (G - 1);
-            const int st = s_st[s];
+            int s, first, stride;
+            deal(s, first, stride);
+            const int st = s >= 0 ? s_st[s] : SL_EMPTY;
             if (st == SL_ACTIVE || st == SL_BACKTRACK || st == SL_NEEDJ) {
                 const bool active = st == SL_ACTIVE;
                 // committed point: the one evaluated last when it was accepted (ACTIVE), else
@@ -1233,18 +1285,16 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                         dvm = dd.y;
                     }
                 };
-                const int ksh = solo >= 0 ? lg : 0;  // element k -> idx = (k << ksh) + koff
-                const int koff = solo >= 0 ? solo : 0;
                 int rown = -1;
                 double4_32a vcn = make_double4_32a(0.0, 0.0, 0.0, 0.0);
                 double dthn = 0.0, dvmn = 0.0;
-                if (tid < nloop()) fetch((tid << ksh) + koff, rown, vcn, dthn, dvmn);
-                for (int k = tid; k < nloop(); k += NT) {
-                    const int idx = (k << ksh) + koff;
+                if (first < n) fetch((first << lg) + s, rown, vcn, dthn, dvmn);
+                for (int k = first; k < n; k += stride) {
+                    const int idx = (k << lg) + s;
                     const int row = rown;
                     const double4_32a vc = vcn;
                     const double dth = dthn, dvm = dvmn;
-                    if (k + NT < nloop()) fetch(((k + NT) << ksh) + koff, rown, vcn, dthn, dvmn);
+                    if (k + stride < n) fetch(((k + stride) << lg) + s, rown, vcn, dthn, dvmn);
                     if (row < 0) continue;
                     const int bus = idx >> lg;
                     // trial point (nr_klu.cpp:665-669 form_trial): committed + alpha * step
@@ -1306,30 +1356,35 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         if constexpr (TIMED) phase_mark(GBPF_PH, &s_clk, 3);
 
         // ---------------------------------------------------------------- evaluate
-        // Buses are swept in reverse Cuthill-McKee order, so the buses a CTA evaluates at the
-        // same time share their neighbours' state in cache.
-        for (int k = tid; k < nloop(); k += NT) {
-            const int s = solo >= 0 ? solo : k & (G - 1);
-            const int st = s_st[s];
-            if (st != SL_FRESH && st != SL_ACTIVE && st != SL_NEEDJ && st != SL_BACKTRACK) continue;
-            const int bus = __ldg(&P.eval_order[solo >= 0 ? k : k >> lg]);
-            const int row = P.row_of_bus[bus];
-            if (row < 0) continue;
+        // From 16 slots on the rows are swept in reverse Cuthill-McKee order, so that the buses a
+        // CTA evaluates at the same time share their neighbours' state in cache; a warp that
+        // holds more rows takes them in order of length (Cuthill-McKee within a length), so that
+        // its lanes end their loops together (one case of the 2,000-bus grid, double: 0.258 ->
+        // 0.197 ms over five evaluations; 16 x 19,999 buses 2.06 -> 1.34 ms).
+        {
+            int s, first, stride;
+            deal(s, first, stride);
+            const int4* const rows = G < 16 ? P.rows_by_len : P.rows;
+            const int st = s >= 0 ? s_st[s] : SL_EMPTY;
+            if (st == SL_FRESH || st == SL_ACTIVE || st == SL_NEEDJ || st == SL_BACKTRACK)
+        for (int k = first; k < P.nv; k += stride) {
+            const int4 rec = __ldg(&rows[k]);
+            const int bus = rec.x;
             const int c = s_case[s];
             const double2 Ssp = ld_in<RING>(Bt.s_shared ? Bt.S + bus : Bt.S + (size_t)bus * Bt.sS + c);
-            const bool pq = P.bus_pq[bus] != 0;
             const bool pinned = spin[((size_t)bus << lg) + s] != 0;
             EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, c, s_nst[s], s_stk[s], s_stv[s]};
             unsigned long long worst;
             if (st == SL_BACKTRACK)
-                worst = eval_row<0>(ec, bus, s, row, pinned, pq, Ssp, fac64, R, true);
+                worst = eval_row<0>(ec, rec, s, pinned, Ssp, fac64, R, true);
             else if (Bt.mixed && s_jprec[s] && s_nojac[s])  // the mismatch only (lazy Jacobian)
-                worst = eval_row<0>(ec, bus, s, row, pinned, pq, Ssp, fac64, R, true);
+                worst = eval_row<0>(ec, rec, s, pinned, Ssp, fac64, R, true);
             else if (Bt.mixed && s_jprec[s])  // into the buffer the slot's last float factors are not in
-                worst = eval_row<2>(ec, bus, s, row, pinned, pq, Ssp, s_fb[s] ? fac32 : fac32b, R, true);
+                worst = eval_row<2>(ec, rec, s, pinned, Ssp, s_fb[s] ? fac32 : fac32b, R, true);
             else
-                worst = eval_row<1>(ec, bus, s, row, pinned, pq, Ssp, fac64, R, true);
-            atomicMax(&s_res[s], worst);
+                worst = eval_row<1>(ec, rec, s, pinned, Ssp, fac64, R, true);
+            raise_max(&s_res[s], worst);
+        }
         }
         __syncthreads();
         if constexpr (TIMED) phase_mark(GBPF_PH, &s_clk, 4);
@@ -1572,7 +1627,7 @@ __device__ void dc_assemble(const DevPlan& P, const double2* Bx, const double* P
             }
             const double b = Bx ? Bx[k].y : -P.Y[k].y;
             if (!Bx) diag -= b;
-            const int q = P.posmap[k];
+            const int q = P.posmap[k].x;
             if (q >= 0) {
                 if (BLOCKS) fac[q] = make_double4_32a(b, 0.0, 0.0, 0.0);
             } else if (P.row_of_bus[j] < 0) {
@@ -1673,16 +1728,13 @@ __global__ void __launch_bounds__(NTB, 1) start_kernel(const StartJob* jobs) {
         sj.iv0[i] = d2f_fast(t1.z);
     }
     __syncthreads();
-    for (int i = tid; i < P.n; i += NTB) {
-        const int row = P.row_of_bus[i];
-        if (row < 0) continue;
+    for (int i = tid; i < P.nv; i += NTB) {
+        const int4 rec = __ldg(&P.rows_by_len[i]);
         EvalCtx ec{&P, sj.Et0, sj.Ei0, sj.iv0, 0, 0, nullptr, 0, 0, 0, nullptr, nullptr};
         if (sj.mixed)
-            eval_row<2>(ec, i, 0, row, false, P.bus_pq[i] != 0, make_double2(0.0, 0.0),
-                        reinterpret_cast<float4*>(sj.fac1), sj.R0, true);
+            eval_row<2>(ec, rec, 0, false, make_double2(0.0, 0.0), reinterpret_cast<float4*>(sj.fac1), sj.R0, true);
         else
-            eval_row<1>(ec, i, 0, row, false, P.bus_pq[i] != 0, make_double2(0.0, 0.0),
-                        reinterpret_cast<double4_32a*>(sj.fac1), sj.R0, true);
+            eval_row<1>(ec, rec, 0, false, make_double2(0.0, 0.0), reinterpret_cast<double4_32a*>(sj.fac1), sj.R0, true);
     }
     __syncthreads();
     if (sj.mixed)
@@ -1769,11 +1821,10 @@ __global__ void eval_debug_kernel(const DevPlan P, const double2* V, const doubl
         iv32[i] = (float)(1.0 / vm);
     }
     __syncthreads();  // single-CTA launch
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int row = P.row_of_bus[i];
-        if (row < 0) continue;
+    for (int i = threadIdx.x; i < P.nv; i += blockDim.x) {
+        const int4 rec = __ldg(&P.rows[i]);
         EvalCtx ec{&P, Et, Ei, iv32, 0, 0, nullptr, 0, 0, 0, nullptr, nullptr};
-        eval_row<1>(ec, i, 0, row, pin && pin[i], P.bus_pq[i] != 0, Sbus[i], blocks, R, true);
+        eval_row<1>(ec, rec, 0, pin && pin[rec.x], Sbus[rec.x], blocks, R, true);
     }
 }
 
