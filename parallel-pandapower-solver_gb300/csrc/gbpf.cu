@@ -125,10 +125,10 @@ gbpf::ScratchOffsets gbpf::scratch_offsets(int n, int nv, int nblk, int G, bool 
 struct Shape {
     int NT = 0, G = 0, lg = 0, occ = 1;
     double chain_cap = 1.0;  // the schedule's chain segment cap (make_schedule)
-    DBuf dtaskA, dptrA, dtaskC, dptrC, dtaskF, dptrF;
+    DBuf dtaskA, dptrA, dtaskC, dptrC, dtaskF, dptrF, dqtaskA, dqptrA, dqtaskC, dqptrC;
     gbpf::DevPlan dp{};
     ~Shape() {
-        for (DBuf* b : {&dtaskA, &dptrA, &dtaskC, &dptrC, &dtaskF, &dptrF})
+        for (DBuf* b : {&dtaskA, &dptrA, &dtaskC, &dptrC, &dtaskF, &dptrF, &dqtaskA, &dqptrA, &dqtaskC, &dqptrC})
             b->release();
     }
 };
@@ -348,36 +348,43 @@ int get_shape(gbpf_solver* s, int NT, int G, Shape** out) {
     sh->occ = std::max(1, occ);
     const gbpf::Plan& p = s->plan;
     gbpf::Schedule sc;
-    gbpf::make_schedule(p, NT / 32, 32 / G, sc, s->chain_cap);
+    const bool quad = sh->lg <= gbpf::QUAD_LG;  // levels with four lanes a task
+    gbpf::Schedule sq;
+    gbpf::make_schedule(p, NT / 32, 32 / G, sc, s->chain_cap, quad ? &sq : nullptr);
     // DIAG tasks carry the "two real pivots" flag (PQ row) in bit 5 of their code
-    for (size_t t = 0; t < sc.taskA.size() / 4; ++t) {
-        if (sc.taskA[4 * t] >= 0 && (sc.taskA[4 * t + 1] & 3) == gbpf::TK_DIAG) {
-            const int row = sc.taskA[4 * t + 1] >> gbpf::TASK_ROW_SHIFT;
-            if (p.row_pq[row]) sc.taskA[4 * t + 1] |= 32;
+    for (std::vector<int>* tasks : {&sc.taskA, &sq.taskA})
+        for (size_t t = 0; t < tasks->size() / 4; ++t) {
+            int* T = &(*tasks)[4 * t];
+            if (T[0] >= 0 && (T[1] & 3) == gbpf::TK_DIAG && p.row_pq[T[1] >> gbpf::TASK_ROW_SHIFT]) T[1] |= 32;
         }
-    }
-    // the first two pairs of every task inline beside its record (8 ints a task): a worker
-    // fetches them with the record, one step ahead, and starts the task's block loads without
-    // first waiting for its pair list
-    auto with_pairs = [&](const std::vector<int>& tasks) {
-        const size_t nt = tasks.size() / 4;
-        std::vector<int> rec(8 * nt, -1);
+    // the first pairs of every task inline beside its record: a worker fetches them with the
+    // record, one step ahead, and starts the task's block loads without first waiting for its
+    // pair list
+    auto with_pairs = [&](const std::vector<int>& tasks, int inl) {
+        const size_t nt = tasks.size() / 4, len = 4 + 2 * (size_t)inl;
+        std::vector<int> rec(len * nt, -1);
         for (size_t t = 0; t < nt; ++t) {
             const int p0 = tasks[4 * t + 2], p1 = tasks[4 * t + 3];
-            std::copy_n(&tasks[4 * t], 4, &rec[8 * t]);
-            for (int k = 0; k < 2 && p0 + k < p1; ++k) {
-                rec[8 * t + 4 + 2 * k] = p.pairs[2 * (size_t)(p0 + k)];
-                rec[8 * t + 5 + 2 * k] = p.pairs[2 * (size_t)(p0 + k) + 1];
+            std::copy_n(&tasks[4 * t], 4, &rec[len * t]);
+            for (int k = 0; k < inl && p0 + k < p1; ++k) {
+                rec[len * t + 4 + 2 * k] = p.pairs[2 * (size_t)(p0 + k)];
+                rec[len * t + 5 + 2 * k] = p.pairs[2 * (size_t)(p0 + k) + 1];
             }
         }
         return rec;
     };
-    CK(upload(sh->dtaskF, with_pairs(sc.taskF)));
-    CK(upload(sh->dptrF, sc.ptrF));
-    CK(upload(sh->dtaskA, with_pairs(sc.taskA)));
+    CK(upload(sh->dtaskA, with_pairs(sc.taskA, 2)));
     CK(upload(sh->dptrA, sc.ptrA));
-    CK(upload(sh->dtaskC, with_pairs(sc.taskC)));
+    CK(upload(sh->dtaskF, with_pairs(sc.taskF, 2)));
+    CK(upload(sh->dptrF, sc.ptrF));
+    CK(upload(sh->dtaskC, with_pairs(sc.taskC, 2)));
     CK(upload(sh->dptrC, sc.ptrC));
+    if (quad) {
+        CK(upload(sh->dqtaskA, with_pairs(sq.taskA, 4)));
+        CK(upload(sh->dqptrA, sq.ptrA));
+        CK(upload(sh->dqtaskC, with_pairs(sq.taskC, 4)));
+        CK(upload(sh->dqptrC, sq.ptrC));
+    }
     sh->dp = s->dp;
     sh->dp.W = NT / G;
     sh->dp.taskA = sh->dtaskA.as<int4>();
@@ -386,6 +393,21 @@ int get_shape(gbpf_solver* s, int NT, int G, Shape** out) {
     sh->dp.ptrC = sh->dptrC.as<int>();
     sh->dp.taskF = sh->dtaskF.as<int4>();
     sh->dp.ptrF = sh->dptrF.as<int>();
+    sh->dp.qtaskA = sh->dqtaskA.as<int4>();
+    sh->dp.qptrA = sh->dqptrA.as<int>();
+    sh->dp.qtaskC = sh->dqtaskC.as<int4>();
+    sh->dp.qptrC = sh->dqptrC.as<int>();
+    // quad levels: those of at most twice the tasks that the CTA's quads take at once, and
+    // backward of at most as many rows. Measured on 118 to 20,000 buses, 1 and 4 slots: limits
+    // of half to four times these are within 3 % of each other for the factor levels; backward
+    // rows use half their lanes only, and twice the limit is 15 % slower at 4 slots.
+    const int at_once = (NT / 32) * std::max(1, 8 / G);
+    sh->dp.quad_from = p.nlev;
+    sh->dp.quad_to = 0;
+    if (quad) {
+        while (sh->dp.quad_from > 0 && sc.tasks_at[sh->dp.quad_from - 1] <= 2 * at_once) --sh->dp.quad_from;
+        while (sh->dp.quad_to < p.nblev && sc.rows_at[sh->dp.quad_to] <= at_once) ++sh->dp.quad_to;
+    }
     *out = sh.get();
     s->shapes.push_back(std::move(sh));
     return 0;
@@ -549,6 +571,7 @@ int enqueue_launch(gbpf_solver* s, LaunchRes& R, gbpf::Batch& b, long long units
     L.scratch = R.scr->as<char>();
     L.cta_bytes = job.off.total;
     L.timed = b.timers;
+    L.mixed = b.mixed;
     CK(cudaEventRecord(R.e0, R.stream));
     if (b.v0_shared)
         CK(gbpf::launch_v0_table(b.V0, s->n, b.check_v0, R.btab->as<double4_32a>(), b.err, R.stream));
@@ -876,6 +899,7 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     L.njobs = nj;
     L.scratch = g->scr.as<char>();
     L.cta_bytes = cta_bytes;
+    L.mixed = mixed;
     CK(cudaEventRecord(g->e0, g->stream));
     for (int q = 0; q < nj; ++q) {
         const gbpf::Batch& b = hj[q].B;

@@ -21,6 +21,7 @@ enum SlotState : int {
 };
 
 constexpr int MAX_SLOTS = 32;    // cases per CTA (G) upper bound
+constexpr int QUAD_LG = 3;       // up to 2^3 slots a CTA: four lanes per factorization task (lu_quad)
 constexpr int MAX_STAMPS = 32;   // outage-stamp entries per case held in shared memory
 
 // error codes written to Batch::err[0] (first error wins; err[1..2] = bus, case)
@@ -53,6 +54,12 @@ struct DevPlan {
     const int* ptrF;
     const int4* taskC;       // backward substitution
     const int* ptrC;
+    // with at most 2^QUAD_LG slots: the same levels for four lanes a task, 3 x int4 a task (four
+    // pairs inline); a double pass that factors takes them from level quad_from on, and backward
+    // up to quad_to
+    const int4 *qtaskA, *qtaskC;
+    const int *qptrA, *qptrC;
+    int quad_from, quad_to;
     const int2* pairs;
     const uint8_t* row_pq;   // block row is PQ (two real pivots)
     const int* bus_of_row;
@@ -181,6 +188,7 @@ struct Launch {
     int njobs;
     char* scratch;
     unsigned long long cta_bytes;
+    int mixed;               // its jobs' precision (a stream launch's jobs each have their own)
     int timed;               // the instantiation that counts SM cycles per phase (stats[8 .. 13])
     Ring ring;
 };

@@ -459,37 +459,87 @@ __device__ __forceinline__ void mm_sub(B4& acc, const B4& a, const B4& b) {
     acc.w = fmadd(-a.w, b.w, fmadd(-a.z, b.y, acc.w));
 }
 
-// One batched factorization + substitution pass over the slots flagged in `on` (G <= 32).
+// *at = max(*at, v) in shared memory. The value only rises, so a v not above what is read needs
+// no atomic (which for 64 bits is a compare-and-swap loop, and one round of it per lane of the
+// slot where a warp holds several rows).
+__device__ __forceinline__ void raise_max(unsigned long long* at, unsigned long long v) {
+    if (v > *(volatile unsigned long long*)at) atomicMax(at, v);
+}
+__device__ __forceinline__ void lower_min(unsigned long long* at, unsigned long long v) {
+    if (v < *(volatile unsigned long long*)at) atomicMin(at, v);
+}
+
+// Smallest and largest pivot magnitude of a worker's diagonal blocks: a00 and det / a00 of each
+// (the two real pivots of a PQ row).
+template <typename T>
+struct Pivots;
+template <>
+struct Pivots<float> {
+    float lo = FLT_MAX, hi = 0.f;
+    __device__ __forceinline__ void see(float u) {
+        const float v = fabsf(u);
+        lo = fminf(lo, v);
+        hi = (v > hi || v != v) ? v : hi;
+    }
+    __device__ __forceinline__ void see_ratio(float det, float x) { see(det / x); }
+    __device__ __forceinline__ unsigned long long lo_bits() const { return dbits(f2d_fast(lo)); }
+    __device__ __forceinline__ unsigned long long hi_bits() const { return dbits(f2d_fast(hi)); }
+};
+// Doubles are kept as ordered bits, off the FP64 pipe, and the quotient is divided out only where
+// it could move a bound: the high words are a piecewise linear logarithm (off by at most 0.087 in
+// log2 each, so a quotient's is within 0.18 of their difference), and a quotient that they put
+// more than 1/4 inside the range seen so far changes nothing. A division holds the FP64 pipe for
+// some 400 cycles, once per pivot on every level's critical path.
+template <>
+struct Pivots<double> {
+    unsigned long long lo = 0x7fefffffffffffffULL, hi = 0ULL;  // DBL_MAX, 0
+    __device__ __forceinline__ void see(double u) {
+        const unsigned long long b = abs_bits(u);
+        lo = b < lo ? b : lo;
+        hi = b > hi ? b : hi;
+    }
+    __device__ __forceinline__ void see_ratio(double det, double x) {
+        const unsigned d = (unsigned)__double2hiint(det) & 0x7fffffffu, v = (unsigned)__double2hiint(x) & 0x7fffffffu;
+        if (d - 0x100000u < 0x7fe00000u && v - 0x100000u < 0x7fe00000u) {  // both normal and finite
+            const int q = (int)(d >> 1) - (int)(v >> 1) + (1023 << 19);     // (halved: fits an int)
+            if (q - (1 << 17) > (int)(lo >> 33) && q + (1 << 17) < (int)(hi >> 33)) return;
+        }
+        see(det / x);
+    }
+    __device__ __forceinline__ unsigned long long lo_bits() const { return lo; }
+    __device__ __forceinline__ unsigned long long hi_bits() const { return hi; }
+};
+
+// What a pass's levels have in common: the slot of this lane, whether it takes part and whether
+// it factors, and how a warp's lanes are shared out (solo: the CTA's one slot left, all lanes).
+struct LuLane {
+    int lg;            // slots of the job's arrays (log2)
+    int ll;            // slots side by side in a warp (log2; solo 0)
+    int s;
+    bool act, factor, factor_any;
+};
+
+// Levels h0 .. h1 - 1 of the factorization and forward substitution, one lane a task.
 // Every warp runs its program of steps (plan.h, Schedule): worker lane / G of the warp does its
-// task of the step for its G slot lanes; the CTA meets at a barrier after each level, forward
-// and backward. The program is static, so its fetches are taken off the level's critical path:
-// a step's record and first two pairs are fetched one step ahead, across level boundaries, and
-// a level's end one level ahead. Pivot statistics per slot go to smin / smax (as ordered bits).
-// With `solo` a slot index, P is the one-slot schedule and all threads work on that slot. Slots
-// flagged in `chord` keep the factors already in `fac` and run the substitutions only; when
-// every slot of the CTA does (factor_any false), the warps walk the substitution-only programs
-// instead of skipping factor tasks one by one.
-template <typename real, bool TIMED = false>
-__device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const double2* R, typename V4<real>::t2* y,
-                        const int* on, int lg, unsigned long long* smin, unsigned long long* smax,
-                        const int* chord, bool factor_any, typename V4<real>::t* dinv_smem, int solo = -1,
-                        unsigned long long* ph = nullptr, long long* clk = nullptr) {
+// task of the step for its G slot lanes; the CTA meets at a barrier after each level. The program
+// is static, so its fetches are taken off the level's critical path: a step's record and first
+// two pairs are fetched one step ahead, across level boundaries, and a level's end one level
+// ahead. Slots that do not factor keep the factors already in `fac` and run the substitutions
+// only; when no slot of the CTA factors, the warps walk the substitution-only programs instead
+// of skipping factor tasks one by one.
+template <typename real>
+__device__ __forceinline__ void lane_forward(const DevPlan& P, const LuLane& L, typename V4<real>::t* fac, const double2* R,
+                                             typename V4<real>::t2* y, typename V4<real>::t* dinv_smem, Pivots<real>& pv,
+                                             int h0, int h1) {
     using B4 = typename V4<real>::t;
     using B2 = typename V4<real>::t2;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    // solo >= 0: one slot left in the CTA; P then carries the one-slot schedule (a worker per
-    // thread) and every thread works on that slot
-    const int s = solo >= 0 ? solo : lane & ((1 << lg) - 1);
-    const int lgw = solo >= 0 ? 5 : 5 - lg;        // workers per warp (log2), and this lane's worker
-    const int wi = solo >= 0 ? lane : lane >> lg;
-    const int warp = tid >> 5;
-    const bool act = on[s] != 0;
-    const bool factor = !(chord && chord[s]);
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int lg = L.lg, s = L.s;
+    const int lgw = 5 - L.ll, wi = (tid & 31) >> L.ll;  // workers per warp (log2), and this lane's worker
+    const bool act = L.act, factor = L.factor, factor_any = L.factor_any;
     // float passes take each task's first two pairs from its head record (the double pass
     // keeps its registers for the wider blocks)
     constexpr bool HEAD = sizeof(real) == 4;
-    real pmin = sizeof(real) == 4 ? (real)FLT_MAX : (real)DBL_MAX, pmax = 0;
     B4 dinv = z4<B4>();  // the worker's last inverse diagonal block: scales the L column after it
     int t = 0, t1 = 0;  // the warp's step, the end of the level's steps
     int4 next = make_int4(-1, 0, 0, 0), nhead = next;
@@ -499,12 +549,12 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
         if constexpr (HEAD) nhead = __ldg(rec + 1);
     };
     if (act) {
-        const int* ptr = (factor_any ? P.ptrA : P.ptrF) + warp * (P.nlev + 1);
+        const int* ptr = (factor_any ? P.ptrA : P.ptrF) + warp * (P.nlev + 1) + h0;
         t = __ldg(ptr);
         t1 = __ldg(ptr + 1);
         fetch(factor_any ? P.taskA : P.taskF);
     }
-    for (int h = 0; h < P.nlev; ++h) {
+    for (int h = h0; h < h1; ++h) {
         if (act) {
             const int t2 = __ldg((factor_any ? P.ptrA : P.ptrF) + warp * (P.nlev + 1) + h + 2);
             while (t < t1) {
@@ -616,14 +666,8 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
                     // records the pivots (a00 and det / a00) and stores the inverse apart, at
                     // block nblk + row (the Jacobian's diagonal stays for the copies)
                     if (!(task.y & 64)) {
-                        const real u0 = fabs(acc.x);
-                        pmin = fmin(pmin, u0);
-                        pmax = (u0 > pmax || u0 != u0) ? u0 : pmax;
-                        if (task.y & 32) {
-                            const real u1 = fabs(det / acc.x);
-                            pmin = fmin(pmin, u1);
-                            pmax = (u1 > pmax || u1 != u1) ? u1 : pmax;
-                        }
+                        pv.see(acc.x);
+                        if (task.y & 32) pv.see_ratio(det, acc.x);
                         fac[((size_t)(P.nblk + (task.y >> 8)) << lg) + s] = dinv;
                     }
                 } else if (task.y & 8) {  // L block: scaled by its column's inverse diagonal
@@ -642,14 +686,33 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
         }
         __syncthreads();
     }
-    if constexpr (TIMED) phase_mark(ph, clk, 1);
+}
+
+// Levels h0 .. h1 - 1 of the backward substitution, one lane a task.
+template <typename real>
+__device__ __forceinline__ void lane_backward(const DevPlan& P, const LuLane& L, typename V4<real>::t* fac,
+                                              typename V4<real>::t2* y, int h0, int h1) {
+    using B4 = typename V4<real>::t;
+    using B2 = typename V4<real>::t2;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int lg = L.lg, s = L.s;
+    const int lgw = 5 - L.ll, wi = (tid & 31) >> L.ll;
+    const bool act = L.act;
+    constexpr bool HEAD = sizeof(real) == 4;
+    int t = 0, t1 = 0;
+    int4 next = make_int4(-1, 0, 0, 0), nhead = next;
+    auto fetch = [&](const int4* task) {
+        const int4* rec = task + 2 * (((size_t)t << lgw) + wi);
+        next = __ldg(rec);
+        if constexpr (HEAD) nhead = __ldg(rec + 1);
+    };
     if (act) {
-        const int* ptr = P.ptrC + warp * (P.nblev + 1);
+        const int* ptr = P.ptrC + warp * (P.nblev + 1) + h0;
         t = __ldg(ptr);
         t1 = __ldg(ptr + 1);
         fetch(P.taskC);
     }
-    for (int h = 0; h < P.nblev; ++h) {
+    for (int h = h0; h < h1; ++h) {
         if (act) {
             const int t2 = __ldg(P.ptrC + warp * (P.nblev + 1) + h + 2);
             while (t < t1) {
@@ -708,27 +771,235 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
         }
         __syncthreads();
     }
-    if (act) {
-        double dmin, dmax;
-        if constexpr (sizeof(real) == 4) {
-            dmin = f2d_fast((float)pmin);
-            dmax = f2d_fast((float)pmax);
-        } else {
-            dmin = pmin;
-            dmax = pmax;
+}
+
+// Levels with four lanes on one task, one per entry of its 2x2 block, on CTAs of at most 2^QUAD_LG
+// slots (and a CTA's last case). A small CTA has few tasks a level in the narrow levels and waits
+// for each one's chain of instructions; four lanes make that chain a quarter as long -- a pair is
+// two dependent multiply-adds instead of eight, which counts above all in double precision,
+// where an instruction holds its sub-core's FP64 pipe for 64 cycles even if one lane works -- and
+// hold a pair in four registers instead of sixteen, so that four pairs are in flight at once. In
+// the wide levels, which are held by the tasks in flight, one lane a task is the better use of a
+// warp. Entries are formed by the operations of the lane form in its order (the inverse and the
+// scaling exchange entries by shuffles), so results are the same bit for bit. A forward or
+// backward row uses its two row lanes (their neighbours repeat them). The quad programs hold
+// 8 / G tasks a step, their records the first four pairs. Double, factorization and forward
+// substitution of one case over a solve: 118 buses 0.28 -> 0.19 ms, 2,000 buses 0.87 -> 0.68; 744
+// cases of 490 buses (4 slots) 0.86 -> 0.68.
+template <typename real>
+struct Quad {
+    using B2 = typename V4<real>::t2;
+    const DevPlan& P;
+    const LuLane& L;
+    real* fac;
+    real* y;
+    int r, c, wi, lgt;        // this lane's entry of the block; the task of the step, tasks a step (log2)
+    unsigned col, rowx, quad; // lanes of the other column / row; the task's four lanes
+    int t = 0, t1 = 0;
+    int4 next, n01, n23;
+    __device__ __forceinline__ Quad(const DevPlan& P, const LuLane& L, typename V4<real>::t* f, B2* y2)
+        : P(P), L(L), fac(reinterpret_cast<real*>(f)), y(reinterpret_cast<real*>(y2)) {
+        const int lane = threadIdx.x & 31;
+        r = (lane >> (L.ll + 1)) & 1;
+        c = (lane >> L.ll) & 1;
+        wi = lane >> (L.ll + 2);
+        lgt = 3 - L.ll;
+        col = 1u << L.ll;
+        rowx = 2u << L.ll;
+        quad = (1u | 1u << col | 1u << rowx | 1u << (col | rowx)) << (lane & ~(int)(col | rowx));
+    }
+    __device__ __forceinline__ void fetch(const int4* task) {
+        const int4* rec = task + 3 * (((size_t)t << lgt) + wi);
+        next = __ldg(rec);
+        n01 = __ldg(rec + 1);
+        n23 = __ldg(rec + 2);
+    }
+    __device__ __forceinline__ size_t at(int item) const { return ((size_t)item << L.lg) + L.s; }
+    // acc -= (row r of block x) . (b0, b1): for factor tasks column c of block y, for
+    // substitution rows the pair (y0, y1) of row y
+    __device__ __forceinline__ real sum(real acc, int4 task, int4 q01, int4 q23, bool subst) const {
+        auto a_of = [&](int x) { return *reinterpret_cast<const B2*>(fac + 4 * at(x) + 2 * r); };
+        auto b_of = [&](int yb) {
+            B2 b;
+            if (subst) {
+                b = reinterpret_cast<const B2*>(y)[at(yb)];
+            } else {
+                const real* p = fac + 4 * at(yb) + c;
+                b.x = p[0];
+                b.y = p[2];
+            }
+            return b;
+        };
+        auto sub = [&](const B2& a, const B2& b) { acc = fmadd(-a.y, b.y, fmadd(-a.x, b.x, acc)); };
+        for (int p = task.z; p < task.w; p += 4) {
+            const int m = task.w - p;
+            if (p > task.z) {
+                const int2 *q = P.pairs + p, i0 = __ldg(q), i1 = m > 1 ? __ldg(q + 1) : make_int2(0, 0);
+                const int2 i2 = m > 2 ? __ldg(q + 2) : make_int2(0, 0), i3 = m > 3 ? __ldg(q + 3) : make_int2(0, 0);
+                q01 = make_int4(i0.x, i0.y, i1.x, i1.y);
+                q23 = make_int4(i2.x, i2.y, i3.x, i3.y);
+            }
+            // (float: all four in flight; double: two and two, in as many registers)
+            constexpr bool ALL = sizeof(real) == 4;
+            B2 a0 = a_of(q01.x), b0 = b_of(q01.y), a1 = {}, b1 = {}, a2 = {}, b2 = {}, a3 = {}, b3 = {};
+            if (m > 1) {
+                a1 = a_of(q01.z);
+                b1 = b_of(q01.w);
+            }
+            if (!ALL) {
+                sub(a0, b0);
+                if (m > 1) sub(a1, b1);
+            }
+            if (m > 2) {
+                a2 = a_of(q23.x);
+                b2 = b_of(q23.y);
+            }
+            if (m > 3) {
+                a3 = a_of(q23.z);
+                b3 = b_of(q23.w);
+            }
+            if (ALL) {
+                sub(a0, b0);
+                if (m > 1) sub(a1, b1);
+            }
+            if (m > 2) sub(a2, b2);
+            if (m > 3) sub(a3, b3);
         }
-        atomicMin(&smin[s], dbits(dmin));
-        atomicMax(&smax[s], dbits(dmax));
+        return acc;
+    }
+
+    __device__ __forceinline__ void forward(const double2* R2, Pivots<real>& pv, int h0, int h1) {
+        const double* const R = reinterpret_cast<const double*>(R2);
+        const int warp = threadIdx.x >> 5;
+        const bool act = L.act, factor = L.factor;
+        real dinv = 0;  // this lane's entry of the last inverse diagonal block
+        if (act) {
+            const int* ptr = P.qptrA + warp * (P.nlev + 1) + h0;
+            t = __ldg(ptr);
+            t1 = __ldg(ptr + 1);
+            fetch(P.qtaskA);
+        }
+        for (int h = h0; h < h1; ++h) {
+            if (act) {
+                const int t2 = __ldg(P.qptrA + warp * (P.nlev + 1) + h + 2);
+                while (t < t1) {
+                    const int4 task = next, q01 = n01, q23 = n23;
+                    ++t;
+                    fetch(P.qtaskA);
+                    const int kind = task.y & 3;
+                    if (task.x < 0 || (kind != 3 && !factor)) continue;
+                    real acc;
+                    if (kind == 3) {
+                        if (task.y & 128)  // its leading pairs are already summed (TASK_CONT)
+                            acc = y[2 * at(task.x) + r];
+                        else if constexpr (sizeof(real) == 4)
+                            acc = d2f_fast(R[2 * at(task.x) + r]);
+                        else
+                            acc = R[2 * at(task.x) + r];
+                    } else {
+                        acc = (task.y & 16) ? (real)0 : fac[4 * at(task.x) + 2 * r + c];
+                    }
+                    acc = sum(acc, task, q01, q23, kind == 3);
+                    if (kind == 3) {
+                        if (c == 0) y[2 * at(task.x) + r] = acc;
+                    } else if (kind == 0) {  // (entries x y z w of the block; this lane's is acc)
+                        const real v1 = __shfl_xor_sync(quad, acc, col), v2 = __shfl_xor_sync(quad, acc, rowx);
+                        const real v3 = __shfl_xor_sync(quad, acc, col | rowx);
+                        const bool on_diag = r == c;  // lane of x or w: (acc, v3) = (x, w), (v1, v2) = (y, z); else crosswise
+                        const real det = fmadd(on_diag ? acc : v1, on_diag ? v3 : v2,
+                                               -mulr(on_diag ? v1 : acc, on_diag ? v2 : v3));
+                        const real inv = (real)1 / det;
+                        dinv = (on_diag ? v3 : -acc) * inv;
+                        if (!(task.y & 64)) {
+                            if (r + c == 0) {
+                                pv.see(acc);
+                                if (task.y & 32) pv.see_ratio(det, acc);
+                            }
+                            fac[4 * at(P.nblk + (task.y >> 8)) + 2 * r + c] = dinv;
+                        }
+                    } else if (task.y & 8) {
+                        const real va = __shfl_xor_sync(quad, acc, col), vd = __shfl_xor_sync(quad, dinv, rowx);
+                        fac[4 * at(task.x) + 2 * r + c] =
+                            fmadd(c ? va : acc, r ? vd : dinv, mulr(c ? acc : va, r ? dinv : vd));
+                    } else {
+                        fac[4 * at(task.x) + 2 * r + c] = acc;
+                    }
+                }
+                t1 = t2;
+            }
+            __syncthreads();
+        }
+    }
+
+    __device__ __forceinline__ void backward(int h0, int h1) {
+        const int warp = threadIdx.x >> 5;
+        const bool act = L.act;
+        if (act) {
+            const int* ptr = P.qptrC + warp * (P.nblev + 1) + h0;
+            t = __ldg(ptr);
+            t1 = __ldg(ptr + 1);
+            fetch(P.qtaskC);
+        }
+        for (int h = h0; h < h1; ++h) {
+            if (act) {
+                const int t2 = __ldg(P.qptrC + warp * (P.nblev + 1) + h + 2);
+                while (t < t1) {
+                    const int4 task = next, q01 = n01, q23 = n23;
+                    ++t;
+                    fetch(P.qtaskC);
+                    if (task.x < 0) continue;
+                    const B2 d = *reinterpret_cast<const B2*>(fac + 4 * at(task.y) + 2 * r);
+                    const real acc = sum(y[2 * at(task.x) + r], task, q01, q23, true);
+                    const real other = __shfl_xor_sync(quad, acc, rowx);
+                    const real o = fmadd(d.x, r ? other : acc, mulr(d.y, r ? acc : other));
+                    if (c == 0) y[2 * at(task.x) + r] = o;
+                }
+                t1 = t2;
+            }
+            __syncthreads();
+        }
+    }
+};
+
+// One batched factorization + substitution pass over the slots flagged in `on` (G <= 32), forward
+// through the levels and back. Pivot statistics per slot go to smin / smax (as ordered bits).
+// With `solo` a slot index, P is the one-slot schedule and all threads work on that slot. Slots
+// flagged in `chord` keep the factors already in `fac` and run the substitutions only. QUADS: a
+// double pass takes the plan's quad levels (DevPlan::quad_from, quad_to). Float passes take none:
+// they wait for memory rather than for a chain of instructions, and one lane a task has more
+// tasks in flight (one case of the 2,000-bus grid: factor levels 0.43 ms, 0.54 with quads
+// throughout, 0.50 with quads in the narrow levels only).
+template <typename real, bool TIMED = false, bool QUADS = true>
+__device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const double2* R, typename V4<real>::t2* y,
+                        const int* on, int lg, unsigned long long* smin, unsigned long long* smax, const int* chord,
+                        bool factor_any, typename V4<real>::t* dinv_smem, int solo = -1, unsigned long long* ph = nullptr,
+                        long long* clk = nullptr) {
+    LuLane L;
+    L.lg = lg;
+    L.ll = solo >= 0 ? 0 : lg;
+    L.s = solo >= 0 ? solo : (threadIdx.x & 31) & ((1 << lg) - 1);
+    L.act = on[L.s] != 0;
+    L.factor = !(chord && chord[L.s]);
+    L.factor_any = factor_any;
+    Pivots<real> pv;
+    if constexpr (sizeof(real) == 8 && QUADS) {
+        const int hq = factor_any ? P.quad_from : P.nlev;
+        lane_forward<real>(P, L, fac, R, y, dinv_smem, pv, 0, hq);
+        if (hq < P.nlev) Quad<real>(P, L, fac, y).forward(R, pv, hq, P.nlev);
+        if constexpr (TIMED) phase_mark(ph, clk, 1);
+        if (P.quad_to) Quad<real>(P, L, fac, y).backward(0, P.quad_to);
+        lane_backward<real>(P, L, fac, y, P.quad_to, P.nblev);
+    } else {
+        lane_forward<real>(P, L, fac, R, y, dinv_smem, pv, 0, P.nlev);
+        if constexpr (TIMED) phase_mark(ph, clk, 1);
+        lane_backward<real>(P, L, fac, y, 0, P.nblev);
+    }
+    if (L.act) {
+        lower_min(&smin[L.s], pv.lo_bits());
+        raise_max(&smax[L.s], pv.hi_bits());
     }
     __syncthreads();
     if constexpr (TIMED) phase_mark(ph, clk, 2);
-}
-
-// *at = max(*at, v) in shared memory. The value only rises, so a v not above what is read needs
-// no atomic (which for 64 bits is a compare-and-swap loop, and one round of it per lane of the
-// slot where a warp holds several rows).
-__device__ __forceinline__ void raise_max(unsigned long long* at, unsigned long long v) {
-    if (v > *(volatile unsigned long long*)at) atomicMax(at, v);
 }
 
 __device__ __forceinline__ bool pivots_ok(unsigned long long bmin, unsigned long long bmax, double rc) {
@@ -741,7 +1012,12 @@ __device__ __forceinline__ bool pivots_ok(unsigned long long bmin, unsigned long
 // NTB threads per CTA and 1024 / NTB resident CTAs per SM (64 registers per thread in
 // every variant): smaller CTAs let one CTA's latency-bound factorization overlap another's
 // double-precision evaluation on the same SM.
-template <int NTB, bool TIMED, bool RING>
+// PREC: 0 a launch of double jobs, 1 of mixed jobs, 2 each job as it says (stream launches). A
+// double launch's kernel carries no float code and takes the quad levels; in the others a double
+// pass, which their cases rarely take, keeps one lane a task. In one kernel the precisions' loops spill each other's registers (64 a thread): with the
+// quad levels inlined beside the float pass, 8,760 mixed cases of the 2,000-bus grid took 10.2
+// ms instead of 9.4; with every double pass out of line the float loops came out 5-10 % slower.
+template <int NTB, bool TIMED, bool RING, int PREC>
 __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L) {
     const int tid = threadIdx.x;
     const int NT = blockDim.x;
@@ -821,6 +1097,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
     __syncthreads();
     const DevPlan& P = s_plan;
     const Batch& Bt = s_batch;
+    const bool mixed = PREC == 2 ? Bt.mixed != 0 : PREC == 1;
     const int n = P.n;
     const int nG = n << lg;
 
@@ -873,7 +1150,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
     // tol and a bound on the voltage error divided by the grid's |J^-1| estimate). `converged`
     // still means mismatch < tol.
     auto loop_head = [&](int s) {
-        const bool polish = Bt.mixed && Bt.vote_rule == 1;
+        const bool polish = mixed && Bt.vote_rule == 1;
         const bool done = s_nrm[s] < (polish ? Bt.tol_polish : Bt.tol);
         if (s_it[s] >= Bt.max_iter) {
             s_st[s] = SL_FINISH;
@@ -928,7 +1205,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                     s_res[s] = 0ULL;
                     s_it[s] = 0;
                     s_conv[s] = 0;
-                    s_vote[s] = Bt.mixed ? 1 : 0;
+                    s_vote[s] = mixed ? 1 : 0;
                     int nst = 0;
                     if (Bt.ymode == 3) {  // the stamps of the case's outaged branches
                         const int e0 = ld_in<RING>(Bt.out_ptr + c), e1 = ld_in<RING>(Bt.out_ptr + c + 1);
@@ -1102,10 +1379,10 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             double nw = bitsd(s_res[s]);
             if (!(nw < BIG)) nw = BIG;
             s_nrm[s] = nw;
-            s_vote[s] = !Bt.mixed ? 0 : (Bt.vote_rule == 1 ? 1 : (nw > Bt.mixed_switch ? 1 : 0));
+            s_vote[s] = !mixed ? 0 : (Bt.vote_rule == 1 ? 1 : (nw > Bt.mixed_switch ? 1 : 0));
             // (what the start's own pass would have set: the precision of the start's Jacobian --
             // the shared one, float on the mixed path -- and the step count)
-            s_jprec[s] = (Bt.mixed && s_vote[s] == 1) ? 1 : 0;
+            s_jprec[s] = (mixed && s_vote[s] == 1) ? 1 : 0;
             loop_head(s);
             if (s_st[s] == SL_ACTIVE) s_it[s] = 1;
         }
@@ -1114,7 +1391,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         if (tid < G) {
             const int s = tid;
             const bool act = s_st[s] == SL_ACTIVE;
-            const bool f32 = act && Bt.mixed && s_vote[s] == 1 && s_jprec[s] == 1;
+            const bool f32 = act && mixed && s_vote[s] == 1 && s_jprec[s] == 1;
             s_on32[s] = f32;
             s_on64[s] = act && !f32;
             s_reeval[s] = act && !f32 && s_jprec[s] == 1 && !s_first[s];
@@ -1122,12 +1399,14 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             s_pmin[s] = ~0ULL;
             s_pmax[s] = 0ULL;
         }
-        const int any32 = __syncthreads_or(tid < G && s_on32[tid]);
+        const int any32 = PREC == 0 ? 0 : __syncthreads_or(tid < G && s_on32[tid]);
+        if (PREC == 0) __syncthreads();
         if constexpr (TIMED) phase_mark(GBPF_PH, &s_clk, 0);
         // a float step that factors after an evaluation that left the Jacobian out: the
         // Jacobian at the same point first (the values that evaluation would have written)
-        const int anylazy = __syncthreads_or(tid < G && s_on32[tid] && !s_nofac[tid] && s_nojac[tid]);
-        if (anylazy) {
+        const int anylazy =
+            PREC == 0 ? 0 : __syncthreads_or(tid < G && s_on32[tid] && !s_nofac[tid] && s_nojac[tid]);
+        if (PREC != 0 && anylazy) {
             for (int idx = tid; idx < P.nv << lg; idx += NT) {
                 const int s = idx & (G - 1);
                 if (!(s_on32[s] && !s_nofac[s] && s_nojac[s])) continue;
@@ -1139,7 +1418,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             __syncthreads();
             if (tid < G && s_on32[tid] && !s_nofac[tid] && s_nojac[tid]) atomicAdd(&Bt.stats[7], 1ULL);
         }
-        if (any32) {
+        if (PREC != 0 && any32) {
             // chord and first steps are decided per slot (a result never depends on the other
             // cases of its CTA); the factorization is left out altogether when no float slot
             // of the CTA factors
@@ -1173,8 +1452,8 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                 s_pmax[s] = 0ULL;
             }
         }
-        const int anyre = __syncthreads_or(tid < G && s_reeval[tid]);
-        if (anyre) {  // this step's factorization is double but the Jacobian was built in float
+        const int anyre = PREC == 0 ? 0 : __syncthreads_or(tid < G && s_reeval[tid]);
+        if (PREC != 0 && anyre) {  // this step's factorization is double but the Jacobian was built in float
             for (int idx = tid; idx < nG; idx += NT) {
                 const int s = idx & (G - 1);
                 if (s_reeval[s]) Ei[idx] = recip_nr((s_tb[s] ? Vb1 : Vb0)[idx].x);
@@ -1192,17 +1471,17 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         }
         const int any64 = __syncthreads_or(tid < G && s_on64[tid]);
         if (any64) {
-            if (s_share) {
-                // no double slot of the CTA factors (all take their first step): substitutions only
-                const int all_first = __syncthreads_and(!(tid < G && s_on64[tid]) || s_nofac[tid]);
-                const int sl = solo >= 0 ? solo : (tid & 31) & (G - 1);
-                double4_32a* const fd = s_first[sl] ? (double4_32a*)Bt.fac0 : fac64;
-                lu_pass<double, TIMED>(solo >= 0 ? s_plan1 : P, fd, R, y64, s_on64, lg, s_pmin, s_pmax, s_nofac, !all_first,
-                                s_dinv64, solo, GBPF_PH, &s_clk);
-            } else {
-                lu_pass<double, TIMED>(solo >= 0 ? s_plan1 : P, fac64, R, y64, s_on64, lg, s_pmin, s_pmax, nullptr, true,
-                                s_dinv64, solo, GBPF_PH, &s_clk);
-            }
+            // no double slot of the CTA factors (all take their first step): substitutions only
+            const int* const nofac = s_share ? s_nofac : nullptr;
+            const int all_first = s_share && __syncthreads_and(!(tid < G && s_on64[tid]) || s_nofac[tid]);
+            const int sl = solo >= 0 ? solo : (tid & 31) & (G - 1);
+            double4_32a* const fd = s_first[sl] ? (double4_32a*)Bt.fac0 : fac64;
+            if constexpr (PREC == 0)
+                lu_pass<double, TIMED>(solo >= 0 ? s_plan1 : P, fd, R, y64, s_on64, lg, s_pmin, s_pmax, nofac, !all_first,
+                                       s_dinv64, solo, GBPF_PH, &s_clk);
+            else
+                lu_pass<double, TIMED, false>(solo >= 0 ? s_plan1 : P, fd, R, y64, s_on64, lg, s_pmin, s_pmax, nofac,
+                                              !all_first, s_dinv64, solo, GBPF_PH, &s_clk);
             if (tid < G && s_on64[tid]) {
                 const int s = tid;
                 if (s_nofac[s]) {
@@ -1268,9 +1547,9 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                 const int cb = active ? s_tb[s] : 1 - s_tb[s];
                 const double4_32a* const Vc = cb ? Vb1 : Vb0;
                 double4_32a* const Vt = cb ? Vb0 : Vb1;
-                const bool ystep32 = s_yprec[s] != 0;
+                const bool ystep32 = PREC != 0 && s_yprec[s] != 0;
                 const double alpha = s_alpha[s];
-                const bool next_double = !Bt.mixed || s_vote[s] != 1;  // the next Jacobian is double
+                const bool next_double = !mixed || s_vote[s] != 1;  // the next Jacobian is double
                 auto fetch = [&](int at, int& row, double4_32a& vc, double& dth, double& dvm) {
                     row = P.row_of_bus[at >> lg];
                     vc = Vc[at];
@@ -1321,7 +1600,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                         if (next_double) {
                             const double iv = recip_nr(vm);
                             Ei[idx] = iv;
-                            iv32[idx] = d2f_fast(iv);
+                            if (PREC != 0) iv32[idx] = d2f_fast(iv);
                         } else {
                             iv32[idx] = __frcp_rn(d2f_fast(vm));
                         }
@@ -1337,7 +1616,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         int qual = 1;
         if (tid < G) {
             const int st = s_st[tid];
-            if (st == SL_FRESH || st == SL_ACTIVE || st == SL_NEEDJ) s_jprec[tid] = (Bt.mixed && s_vote[tid] == 1) ? 1 : 0;
+            if (st == SL_FRESH || st == SL_ACTIVE || st == SL_NEEDJ) s_jprec[tid] = (mixed && s_vote[tid] == 1) ? 1 : 0;
             if (st == SL_ACTIVE && s_jprec[tid])
                 qual = Bt.lazy_jac && (s_chord[tid] || s_nrm[tid] < JAC_LAZY * Bt.chord_tol);
             s_res[tid] = 0ULL;
@@ -1374,15 +1653,14 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             const double2 Ssp = ld_in<RING>(Bt.s_shared ? Bt.S + bus : Bt.S + (size_t)bus * Bt.sS + c);
             const bool pinned = spin[((size_t)bus << lg) + s] != 0;
             EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, c, s_nst[s], s_stk[s], s_stv[s]};
-            unsigned long long worst;
-            if (st == SL_BACKTRACK)
+            unsigned long long worst = 0ULL;
+            if (st == SL_BACKTRACK || (mixed && s_jprec[s] && s_nojac[s]))  // the mismatch only (line search, lazy Jacobian)
                 worst = eval_row<0>(ec, rec, s, pinned, Ssp, fac64, R, true);
-            else if (Bt.mixed && s_jprec[s] && s_nojac[s])  // the mismatch only (lazy Jacobian)
-                worst = eval_row<0>(ec, rec, s, pinned, Ssp, fac64, R, true);
-            else if (Bt.mixed && s_jprec[s])  // into the buffer the slot's last float factors are not in
-                worst = eval_row<2>(ec, rec, s, pinned, Ssp, s_fb[s] ? fac32 : fac32b, R, true);
-            else
+            else if (PREC != 0 && mixed && s_jprec[s]) {  // into the buffer the slot's last float factors are not in
+                if constexpr (PREC != 0) worst = eval_row<2>(ec, rec, s, pinned, Ssp, s_fb[s] ? fac32 : fac32b, R, true);
+            } else {
                 worst = eval_row<1>(ec, rec, s, pinned, Ssp, fac64, R, true);
+            }
             raise_max(&s_res[s], worst);
         }
         }
@@ -1406,14 +1684,14 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             // from below mixed_switch that does not halve the mismatch, or needs damping).
             if (st == SL_FRESH) {
                 s_nrm[s] = nw;
-                s_vote[s] = !Bt.mixed ? 0 : (Bt.vote_rule == 1 ? 1 : (nw > Bt.mixed_switch ? 1 : 0));
+                s_vote[s] = !mixed ? 0 : (Bt.vote_rule == 1 ? 1 : (nw > Bt.mixed_switch ? 1 : 0));
                 top = true;
             } else if (st == SL_ACTIVE) {
                 const double old = s_nrm[s];
                 const bool was_chord = s_chord[s] != 0;
                 s_chord[s] = 0;
                 if (!Bt.line_search || nw <= (1.0 - ARMIJO_C) * old) {
-                    if (Bt.mixed && s_vote[s] >= 0) {
+                    if (mixed && s_vote[s] >= 0) {
                         if (Bt.vote_rule == 1) {
                             // (a chord step that contracts poorly only means: refactor next)
                             if (!was_chord && s_vote[s] == 1 && !(nw <= 0.5 * old) && old < Bt.mixed_switch)
@@ -1439,7 +1717,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                     s_alpha[s] = 0.5;
                     s_trial[s] = 1;
                     s_st[s] = SL_BACKTRACK;
-                    if (Bt.mixed && (Bt.vote_rule == 0 || old < Bt.mixed_switch)) s_vote[s] = -1;
+                    if (mixed && (Bt.vote_rule == 0 || old < Bt.mixed_switch)) s_vote[s] = -1;
                 }
             } else if (st == SL_BACKTRACK) {
                 const double a = s_alpha[s];
@@ -1741,8 +2019,7 @@ __global__ void __launch_bounds__(NTB, 1) start_kernel(const StartJob* jobs) {
         lu_pass<float>(P, reinterpret_cast<float4*>(sj.fac1), sj.R0, reinterpret_cast<float2*>(sj.y0), s_on, 0, s_min,
                        s_max, nullptr, true, nullptr);
     else
-        lu_pass<double>(P, reinterpret_cast<double4_32a*>(sj.fac1), sj.R0, sj.y0, s_on, 0, s_min, s_max, nullptr, true,
-                        nullptr);
+        lu_pass<double>(P, reinterpret_cast<double4_32a*>(sj.fac1), sj.R0, sj.y0, s_on, 0, s_min, s_max, nullptr, true, nullptr);
     if (tid == 0) *sj.ok0 = pivots_ok(s_min[0], s_max[0], sj.rcond_min) ? 1 : 0;
 }
 
@@ -1828,24 +2105,31 @@ __global__ void eval_debug_kernel(const DevPlan P, const double2* V, const doubl
     }
 }
 
+template <int NTB>
+static void start_newton(const Launch& L, int grid, cudaStream_t stream) {
+    if (L.mixed)
+        L.timed ? newton_kernel<NTB, true, false, 1><<<grid, NTB, 0, stream>>>(L)
+                : newton_kernel<NTB, false, false, 1><<<grid, NTB, 0, stream>>>(L);
+    else
+        L.timed ? newton_kernel<NTB, true, false, 0><<<grid, NTB, 0, stream>>>(L)
+                : newton_kernel<NTB, false, false, 0><<<grid, NTB, 0, stream>>>(L);
+}
+
 cudaError_t launch_newton(const Launch& L, int grid, int threads, cudaStream_t stream) {
     if (L.ring.published) {  // a stream launch: untimed
         if (L.timed) return cudaErrorInvalidValue;
         if (threads == 1024)
-            newton_kernel<1024, false, true><<<grid, 1024, 0, stream>>>(L);
+            newton_kernel<1024, false, true, 2><<<grid, 1024, 0, stream>>>(L);
         else if (threads == 512)
-            newton_kernel<512, false, true><<<grid, 512, 0, stream>>>(L);
+            newton_kernel<512, false, true, 2><<<grid, 512, 0, stream>>>(L);
         else
             return cudaErrorInvalidValue;
     } else if (threads == 1024)
-        L.timed ? newton_kernel<1024, true, false><<<grid, 1024, 0, stream>>>(L)
-                : newton_kernel<1024, false, false><<<grid, 1024, 0, stream>>>(L);
+        start_newton<1024>(L, grid, stream);
     else if (threads == 512)
-        L.timed ? newton_kernel<512, true, false><<<grid, 512, 0, stream>>>(L)
-                : newton_kernel<512, false, false><<<grid, 512, 0, stream>>>(L);
+        start_newton<512>(L, grid, stream);
     else if (threads == 256)
-        L.timed ? newton_kernel<256, true, false><<<grid, 256, 0, stream>>>(L)
-                : newton_kernel<256, false, false><<<grid, 256, 0, stream>>>(L);
+        start_newton<256>(L, grid, stream);
     else
         return cudaErrorInvalidValue;
     return cudaGetLastError();
@@ -1859,9 +2143,9 @@ cudaError_t launch_eval_debug(const DevPlan& P, const double2* V, const double2*
 }
 
 const void* newton_kernel_ptr(int threads) {
-    if (threads == 1024) return (const void*)newton_kernel<1024, false, false>;
-    if (threads == 512) return (const void*)newton_kernel<512, false, false>;
-    return (const void*)newton_kernel<256, false, false>;
+    if (threads == 1024) return (const void*)newton_kernel<1024, false, false, 0>;
+    if (threads == 512) return (const void*)newton_kernel<512, false, false, 0>;
+    return (const void*)newton_kernel<256, false, false, 0>;
 }
 
 }  // namespace gbpf

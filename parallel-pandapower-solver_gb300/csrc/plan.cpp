@@ -548,10 +548,9 @@ std::vector<Task> cut_long(const Plan& p, std::vector<Task> tasks, int nlev, int
 
 }  // namespace
 
-void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double chain_cap) {
+void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double chain_cap, Schedule* quad) {
     out.nwarps = std::max(1, nwarps);
     out.wpw = std::max(1, wpw);
-    out.level_work.assign(std::max(p.nlev, p.nblev), 0);
     // factor-level key: the task's destination block (a forward row: its diagonal block)
     auto keys = [&](const std::vector<Task>& tasks, bool rows) {
         std::vector<int> key(tasks.size());
@@ -565,10 +564,23 @@ void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double cha
     const int workers = out.nwarps * out.wpw;
     const std::vector<Task> A = cut_long(p, p.tasksA, p.nlev, workers);
     fwd = cut_long(p, fwd, p.nlev, workers);
-    layout(A, p.nlev, out.nwarps, out.wpw, out.taskA, out.ptrA, &out.level_work, keys(A, false), chain_cap, true);
-    layout(fwd, p.nlev, out.nwarps, out.wpw, out.taskF, out.ptrF, nullptr, keys(fwd, false), chain_cap, false);
-    layout(p.tasksC, p.nblev, out.nwarps, out.wpw, out.taskC, out.ptrC, nullptr, keys(p.tasksC, true), chain_cap,
-           false);
+    const std::vector<int> keyA = keys(A, false), keyF = keys(fwd, false), keyC = keys(p.tasksC, true);
+    auto lay = [&](Schedule& sc) {
+        sc.level_work.assign(std::max(p.nlev, p.nblev), 0);
+        layout(A, p.nlev, sc.nwarps, sc.wpw, sc.taskA, sc.ptrA, &sc.level_work, keyA, chain_cap, true);
+        layout(fwd, p.nlev, sc.nwarps, sc.wpw, sc.taskF, sc.ptrF, nullptr, keyF, chain_cap, false);
+        layout(p.tasksC, p.nblev, sc.nwarps, sc.wpw, sc.taskC, sc.ptrC, nullptr, keyC, chain_cap, false);
+    };
+    lay(out);
+    if (quad) {
+        quad->nwarps = out.nwarps;
+        quad->wpw = out.wpw / 4;
+        lay(*quad);
+    }
+    out.tasks_at.assign(p.nlev, 0);
+    out.rows_at.assign(p.nblev, 0);
+    for (const Task& t : A) ++out.tasks_at[t.level];
+    for (const Task& t : p.tasksC) ++out.rows_at[t.level];
 }
 
 // ----------------------------------------------------------------------------- host replica

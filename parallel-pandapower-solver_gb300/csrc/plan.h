@@ -58,6 +58,7 @@ struct Schedule {
     std::vector<int> taskF, ptrF;   // the forward substitution alone (chord passes)
     std::vector<int> taskC, ptrC;   // backward substitution
     std::vector<int> level_work;    // per level: max worker load
+    std::vector<int> tasks_at, rows_at;  // tasks of every factor level, rows of every backward level
 };
 
 struct Plan {
@@ -108,8 +109,9 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
 // Deal the plan's tasks to `nwarps` warps of `wpw` workers (longest first onto the least-loaded
 // warp); a level's diagonal-and-L chain heavier than chain_cap x the level's mean work per
 // worker is cut into segments on different workers, each later one recomputing the diagonal
-// inverse (0: chains are never cut).
-void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double chain_cap = 1.0);
+// inverse (0: chains are never cut). `quad`: the same tasks dealt once more for four lanes a
+// task (wpw / 4 tasks a step), or null.
+void make_schedule(const Plan& p, int nwarps, int wpw, Schedule& out, double chain_cap = 1.0, Schedule* quad = nullptr);
 
 // Host replica of the device algorithm (double precision): Jacobian blocks at (Vm, Va)
 // written to `blocks` (nblk*4, zero where not in the Jacobian) and residual R (nv*2).

@@ -1,0 +1,35 @@
+"""Launches of few cases per CTA on the GPU, where one lane or four work on a factorization task:
+grids around the sizes where levels change over, 1 to 8 slots a CTA, both precisions. Every
+CTA shape forms the same numbers, so a case's result must be bit-identical whatever its launch,
+and within the double path's 1e-11 of the oracle."""
+
+import numpy as np
+import pytest
+
+from oracle import cpu
+from p3s_gb300.solver import GpuSolver
+from p3s_gb300.synthetic import make_grid, scenario_injections
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [5, 30, 65, 257, 1031])
+def test_small_shapes_agree_bit_for_bit(n):
+    g = make_grid(n, seed=n, max_drop_pu=0.05)
+    S = scenario_injections(g, 13, seed=n)
+    ref = cpu.Solver(g.Yp, g.Yj, g.Yx, g.pv, g.pq).solve_batch(S, g.V0)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    # (the reference's votes take every mixed case through a double Jacobian and factorization)
+    for precision, rule in (("double", "gb300"), ("mixed", "gb300"), ("mixed", "reference")):
+        p = GpuSolver.params(precision=precision, vote_rule=rule)
+        first = None
+        for nt, slots in ((1024, 1), (1024, 4), (512, 1), (512, 2), (512, 8), (256, 4), (512, 16), (512, 32)):
+            s.set_shape(13, nt, slots)
+            r = s.solve_batch(S, g.V0, p)
+            if first is None:
+                first = r
+            assert np.array_equal(r["V"], first["V"]) and np.array_equal(r["iterations"], first["iterations"])
+        assert np.array_equal(first["converged"], ref["converged"]) and ref["converged"].all()
+        if precision == "double":
+            assert np.array_equal(first["iterations"], ref["iterations"])
+            assert np.abs(first["V"] - ref["V"]).max() < 1e-11
