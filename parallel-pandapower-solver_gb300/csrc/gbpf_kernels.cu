@@ -96,6 +96,18 @@ __device__ __forceinline__ float d2f_trunc(double d) {
     return __uint_as_float((hi & 0x80000000u) | (a >= (897u << 20) ? m : 0u));
 }
 
+// One slot's items of a [item][slot] array (2^lg slots): the slot is in the base and the item's
+// offset one widening multiply-add, where shifting and adding the slot take five or six.
+template <typename T>
+struct Slots {
+    T* base;
+    unsigned step;
+    __device__ __forceinline__ Slots(T* array, int s, int lg) : base(array + s), step((unsigned)sizeof(T) << lg) {}
+    __device__ __forceinline__ T& operator[](int item) const {
+        return *(T*)((char*)base + (unsigned long long)(unsigned)item * step);
+    }
+};
+
 // |x| as ordered bits (sign cleared): compares like the magnitudes, NaN above everything
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
     return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
@@ -210,11 +222,11 @@ __device__ __forceinline__ double2 less_stamps(const EvalCtx& c, double2 y, int 
     return y;
 }
 
-__device__ __forceinline__ void put_block(double4_32a* fac, size_t at, double a, double b, double c, double d) {
-    fac[at] = make_double4_32a(a, b, c, d);
+__device__ __forceinline__ void put_block(double4_32a& blk, double a, double b, double c, double d) {
+    blk = make_double4_32a(a, b, c, d);
 }
-__device__ __forceinline__ void put_block(float4* fac, size_t at, double a, double b, double c, double d) {
-    fac[at] = make_float4((float)a, (float)b, (float)c, (float)d);
+__device__ __forceinline__ void put_block(float4& blk, double a, double b, double c, double d) {
+    blk = make_float4((float)a, (float)b, (float)c, (float)d);
 }
 
 // A row's record (DevPlan::rows): bus, block row, first nonzero, nonzeros << 1 | PQ.
@@ -225,12 +237,13 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
     const int i = rec.x, row = rec.y;
     const int k0 = rec.z, k1 = rec.z + (rec.w >> 1);
     const bool pq_i = rec.w & 1;
-    const size_t si = ((size_t)i << c.lg) + s;
-    const double2 ei = c.Et[si];
+    const Slots<const double2> Et(c.Et, s, c.lg);
+    const Slots<FacT> F(fac, s, c.lg);
+    const double2 ei = Et[i];
     // float copy of the evaluation point for the float Jacobian: (e, f) truncated from the
     // double phasor, 1 / Vm from its float array (read for PQ buses only)
     float4 vi32 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (JM == 2) vi32 = make_float4(d2f_trunc(ei.x), d2f_trunc(ei.y), pq_i ? c.iv32[si] : 0.f, 0.f);
+    if (JM == 2) vi32 = make_float4(d2f_trunc(ei.x), d2f_trunc(ei.y), pq_i ? Slots<const float>(c.iv32, s, c.lg)[i] : 0.f, 0.f);
     double Ir = 0.0, Ii = 0.0, gii = 0.0, bii = 0.0;
     float gii32 = 0.f, bii32 = 0.f;
     const unsigned mask = row_stamp_mask(c, k0, k1);
@@ -243,7 +256,7 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
         jn = __ldg(&P.Yj[k0]);
         yn = ybus_load(c, k0);
         jn2 = __ldg(&P.Yj[min(k0 + 1, k1 - 1)]);
-        en = c.Et[((size_t)jn << c.lg) + s];
+        en = Et[jn];
     }
     for (int k = k0; k < k1; ++k) {
         const int j = jn;
@@ -251,11 +264,10 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
         const double2 y = less_stamps(c, yn, k, mask);
         if (k + 1 < k1) {
             jn = jn2;
-            en = c.Et[((size_t)jn << c.lg) + s];
+            en = Et[jn];
             yn = ybus_load(c, k + 1);
             jn2 = __ldg(&P.Yj[min(k + 2, k1 - 1)]);
         }
-        const size_t sj = ((size_t)j << c.lg) + s;
         Ir = fma(y.x, ej.x, Ir);
         Ir = fma(-y.y, ej.y, Ir);
         Ii = fma(y.x, ej.y, Ii);
@@ -280,16 +292,15 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
         const int q = qj.x;
         if (q < 0) continue;
         const bool pq_j = qj.y != 0;
-        const size_t at = ((size_t)q << c.lg) + s;
         if (pinned) {
-            put_block(fac, at, 0.0, 0.0, 0.0, 0.0);
+            put_block(F[q], 0.0, 0.0, 0.0, 0.0);
             continue;
         }
         if (JM == 1) {
             const double wr = fma(-y.y, ej.y, y.x * ej.x), wi = fma(y.y, ej.x, y.x * ej.y);
             const double Wr = fma(ei.x, wr, ei.y * wi), Wi = fma(ei.y, wr, -ei.x * wi);
-            const double ivj = c.Ei[sj];
-            put_block(fac, at, Wi, pq_j ? Wr * ivj : 0.0, pq_i ? -Wr : 0.0, (pq_i && pq_j) ? Wi * ivj : 0.0);
+            const double ivj = Slots<const double>(c.Ei, s, c.lg)[j];
+            put_block(F[q], Wi, pq_j ? Wr * ivj : 0.0, pq_i ? -Wr : 0.0, (pq_i && pq_j) ? Wi * ivj : 0.0);
         } else {
             float gx, gy;
             if (c.ymode == 0) {
@@ -300,28 +311,28 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
                 gx = d2f_fast(y.x);
                 gy = d2f_fast(y.y);
             }
-            const float4 vj = make_float4(d2f_trunc(ej.x), d2f_trunc(ej.y), pq_j ? c.iv32[sj] : 0.f, 0.f);
+            const float4 vj = make_float4(d2f_trunc(ej.x), d2f_trunc(ej.y), pq_j ? Slots<const float>(c.iv32, s, c.lg)[j] : 0.f, 0.f);
             const float wr = fmaf(-gy, vj.y, gx * vj.x), wi = fmaf(gy, vj.x, gx * vj.y);
             const float Wr = fmaf(vi32.x, wr, vi32.y * wi), Wi = fmaf(vi32.y, wr, -vi32.x * wi);
-            reinterpret_cast<float4*>(fac)[at] =
+            reinterpret_cast<float4&>(F[q]) =
                 make_float4(Wi, pq_j ? Wr * vj.z : 0.f, pq_i ? -Wr : 0.f, (pq_i && pq_j) ? Wi * vj.z : 0.f);
         }
     }
     const double Pc = fma(ei.x, Ir, ei.y * Ii);
     const double Qc = fma(ei.y, Ir, -ei.x * Ii);
     if (JM == 1) {
-        const size_t at = ((size_t)P.dpos[row] << c.lg) + s;
+        FacT& diag = F[P.dpos[row]];
         if (pinned) {
-            put_block(fac, at, 1.0, 0.0, 0.0, 1.0);
+            put_block(diag, 1.0, 0.0, 0.0, 1.0);
         } else {
             const double vi2 = fma(ei.x, ei.x, ei.y * ei.y);
             const double Ps = vi2 * gii, Qs = -vi2 * bii;
-            const double ivi = c.Ei[si];
-            put_block(fac, at, Qs - Qc, pq_i ? (Pc + Ps) * ivi : 0.0, pq_i ? Pc - Ps : 0.0,
+            const double ivi = Slots<const double>(c.Ei, s, c.lg)[i];
+            put_block(diag, Qs - Qc, pq_i ? (Pc + Ps) * ivi : 0.0, pq_i ? Pc - Ps : 0.0,
                       pq_i ? (Qc + Qs) * ivi : 1.0);
         }
     } else if (JM == 2) {  // float diagonal block from float copies: no double arithmetic
-        const size_t at = ((size_t)P.dpos[row] << c.lg) + s;
+        FacT& diag = F[P.dpos[row]];
         float4 o;
         if (pinned) {
             o = make_float4(1.f, 0.f, 0.f, 1.f);
@@ -332,11 +343,11 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
             o = make_float4(Qs - Q32, pq_i ? (P32 + Ps) * vi32.z : 0.f, pq_i ? P32 - Ps : 0.f,
                             pq_i ? (Q32 + Qs) * vi32.z : 1.f);
         }
-        reinterpret_cast<float4*>(fac)[at] = o;
+        reinterpret_cast<float4&>(diag) = o;
     }
     const double rp = pinned ? 0.0 : Ssp.x - Pc;
     const double rq = (pinned || !pq_i) ? 0.0 : Ssp.y - Qc;
-    if (write_r) R[((size_t)row << c.lg) + s] = make_double2(rp, rq);
+    if (write_r) Slots<double2>(R, s, c.lg)[row] = make_double2(rp, rq);
     const unsigned long long a = abs_bits(rp), b = abs_bits(rq);
     return b > a ? b : a;
 }
@@ -791,19 +802,21 @@ struct Quad {
     using B2 = typename V4<real>::t2;
     const DevPlan& P;
     const LuLane& L;
-    real* fac;
-    real* y;
+    real *fa, *fb, *y;        // the slot's first block from (r, 0) and (0, c) on, its first pair
+    unsigned step;            // bytes from block to block
     int r, c, wi, lgt;        // this lane's entry of the block; the task of the step, tasks a step (log2)
     unsigned col, rowx, quad; // lanes of the other column / row; the task's four lanes
     int t = 0, t1 = 0;
     int4 next, n01, n23;
     __device__ __forceinline__ Quad(const DevPlan& P, const LuLane& L, typename V4<real>::t* f, B2* y2)
-        : P(P), L(L), fac(reinterpret_cast<real*>(f)), y(reinterpret_cast<real*>(y2)) {
+        : P(P), L(L), y(reinterpret_cast<real*>(y2 + L.s)), step((unsigned)(4 * sizeof(real)) << L.lg) {
         const int lane = threadIdx.x & 31;
         r = (lane >> (L.ll + 1)) & 1;
         c = (lane >> L.ll) & 1;
         wi = lane >> (L.ll + 2);
         lgt = 3 - L.ll;
+        fa = reinterpret_cast<real*>(f + L.s) + 2 * r;
+        fb = reinterpret_cast<real*>(f + L.s) + c;
         col = 1u << L.ll;
         rowx = 2u << L.ll;
         quad = (1u | 1u << col | 1u << rowx | 1u << (col | rowx)) << (lane & ~(int)(col | rowx));
@@ -814,17 +827,28 @@ struct Quad {
         n01 = __ldg(rec + 1);
         n23 = __ldg(rec + 2);
     }
-    __device__ __forceinline__ size_t at(int item) const { return ((size_t)item << L.lg) + L.s; }
+    // row r of a block, entry (0, c) of a block, component r of a row's pair
+    __device__ __forceinline__ B2& row_of(int x) const {
+        return *(B2*)((char*)fa + (unsigned long long)(unsigned)x * step);
+    }
+    __device__ __forceinline__ real* col_of(int x) const {
+        return (real*)((char*)fb + (unsigned long long)(unsigned)x * step);
+    }
+    __device__ __forceinline__ real& entry(int x) const { return reinterpret_cast<real*>(&row_of(x))[c]; }
+    __device__ __forceinline__ B2& pair(int x) const {
+        return *(B2*)((char*)y + (unsigned long long)(unsigned)x * (step / 2));
+    }
+    __device__ __forceinline__ real& comp(int x) const { return reinterpret_cast<real*>(&pair(x))[r]; }
     // acc -= (row r of block x) . (b0, b1): for factor tasks column c of block y, for
     // substitution rows the pair (y0, y1) of row y
     __device__ __forceinline__ real sum(real acc, int4 task, int4 q01, int4 q23, bool subst) const {
-        auto a_of = [&](int x) { return *reinterpret_cast<const B2*>(fac + 4 * at(x) + 2 * r); };
+        auto a_of = [&](int x) { return row_of(x); };
         auto b_of = [&](int yb) {
             B2 b;
             if (subst) {
-                b = reinterpret_cast<const B2*>(y)[at(yb)];
+                b = pair(yb);
             } else {
-                const real* p = fac + 4 * at(yb) + c;
+                const real* p = col_of(yb);
                 b.x = p[0];
                 b.y = p[2];
             }
@@ -891,17 +915,17 @@ struct Quad {
                     real acc;
                     if (kind == 3) {
                         if (task.y & 128)  // its leading pairs are already summed (TASK_CONT)
-                            acc = y[2 * at(task.x) + r];
+                            acc = comp(task.x);
                         else if constexpr (sizeof(real) == 4)
-                            acc = d2f_fast(R[2 * at(task.x) + r]);
+                            acc = d2f_fast(R[2 * (((size_t)task.x << L.lg) + L.s) + r]);
                         else
-                            acc = R[2 * at(task.x) + r];
+                            acc = R[2 * (((size_t)task.x << L.lg) + L.s) + r];
                     } else {
-                        acc = (task.y & 16) ? (real)0 : fac[4 * at(task.x) + 2 * r + c];
+                        acc = (task.y & 16) ? (real)0 : entry(task.x);
                     }
                     acc = sum(acc, task, q01, q23, kind == 3);
                     if (kind == 3) {
-                        if (c == 0) y[2 * at(task.x) + r] = acc;
+                        if (c == 0) comp(task.x) = acc;
                     } else if (kind == 0) {  // (entries x y z w of the block; this lane's is acc)
                         const real v1 = __shfl_xor_sync(quad, acc, col), v2 = __shfl_xor_sync(quad, acc, rowx);
                         const real v3 = __shfl_xor_sync(quad, acc, col | rowx);
@@ -915,14 +939,14 @@ struct Quad {
                                 pv.see(acc);
                                 if (task.y & 32) pv.see_ratio(det, acc);
                             }
-                            fac[4 * at(P.nblk + (task.y >> 8)) + 2 * r + c] = dinv;
+                            entry(P.nblk + (task.y >> 8)) = dinv;
                         }
                     } else if (task.y & 8) {
                         const real va = __shfl_xor_sync(quad, acc, col), vd = __shfl_xor_sync(quad, dinv, rowx);
-                        fac[4 * at(task.x) + 2 * r + c] =
+                        entry(task.x) =
                             fmadd(c ? va : acc, r ? vd : dinv, mulr(c ? acc : va, r ? dinv : vd));
                     } else {
-                        fac[4 * at(task.x) + 2 * r + c] = acc;
+                        entry(task.x) = acc;
                     }
                 }
                 t1 = t2;
@@ -948,11 +972,11 @@ struct Quad {
                     ++t;
                     fetch(P.qtaskC);
                     if (task.x < 0) continue;
-                    const B2 d = *reinterpret_cast<const B2*>(fac + 4 * at(task.y) + 2 * r);
-                    const real acc = sum(y[2 * at(task.x) + r], task, q01, q23, true);
+                    const B2 d = row_of(task.y);
+                    const real acc = sum(comp(task.x), task, q01, q23, true);
                     const real other = __shfl_xor_sync(quad, acc, rowx);
                     const real o = fmadd(d.x, r ? other : acc, mulr(d.y, r ? acc : other));
-                    if (c == 0) y[2 * at(task.x) + r] = o;
+                    if (c == 0) comp(task.x) = o;
                 }
                 t1 = t2;
             }
