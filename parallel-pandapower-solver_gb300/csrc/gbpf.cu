@@ -300,13 +300,75 @@ int size_class(long long units) {
     return c;
 }
 
-// CTA shape for a batch of `units` work items. Case slots per SM: the batch's share of an
-// SM rounded up to a power of two (measured on GB300, 2,000-bus grid: every batch from 1 to
-// 8,760 cases is within a few percent of its best shape this way), at most 64 per SM
-// (32 per SM above 4,096 variable buses, 16 above 16,384: the per-slot working set grows
-// with the grid). Up to 4 slots per SM run as one 1,024-thread CTA (many workers per
-// case); more run as two 512-thread CTAs per SM, whose phases overlap.
-void choose_shape(const gbpf_solver* s, long long units, int* NT, int* G) {
+// CTA shape for a batch of `units` cases of one grid (measured on GB300, 118 to 3,500 buses, 700
+// to 8,760 cases). Case slots per SM: the batch's share of an SM rounded up to a power of two, at
+// most 64 (32 above 4,096 variable buses, 16 above 16,384: the per-slot working set grows with the
+// grid). Up to 4 slots per SM run as one 1,024-thread CTA (many workers per case), more as two
+// 512-thread CTAs whose phases overlap -- except:
+// * mixed, 8 to 32 slots per SM on larger grids (from 24,000 buses x slots on): one 1,024-thread
+//   CTA. Twice the workers on one slot set shorten the waits that bound a pass there (2,000 buses,
+//   3,001 cases: 5.25 -> 4.93 ms; 3,500 buses, 2,432 cases 5.1 -> 4.6), below it they are equal.
+// * mixed, 8 to 32 slots per SM of which at most three quarters are needed: three of four
+//   256-thread CTAs (490 buses, 744 cases 0.85 -> 0.83 ms, 3,001 cases 1.67 -> 1.60).
+// * double: the FP64 pipes are the bound, and they take a warp's time for however few of its
+//   lanes work, so a rounded-up share is paid for in full. The shape with the fewest slots on
+//   the fullest SM: CTAs not all resident at once are refilled and share the cases evenly, at
+//   the price of about one more CTA's slots at the end (on grids below 400 buses of far more);
+//   32-slot CTAs (a worker a warp, no divergence) do a slot's work in 0.84 of the time, 4- and
+//   2-slot ones in 1.12 and 1.25, and eight slots in all leave an SM waiting; one CTA of fewer
+//   than 1,024 threads alone on its SM takes 1.05. 2,000 buses: 744 cases 3.58 -> 3.14 ms, 3,001
+//   cases 10.7 -> 8.6, 6,000 cases 17.8 -> 14.0; 490 buses, 3,001 cases 3.1 -> 2.6.
+// * outage cases take unlike numbers of passes, so slots that refill pay more: double counts
+//   half a CTA's slots on top, and a CTA holds at most 8,192 buses x slots (2,000-bus N-1 sweep:
+//   mixed 14.4 -> 13.3 ms, double 25.0 -> 23.1; 1,000 buses 3.2 -> 3.1 and 6.1 -> 5.1).
+void batch_shape(int nsm, int nv, long long units, bool mixed, bool outages, int* NT, int* G) {
+    const int cap = nv <= 4096 ? 64 : (nv <= 16384 ? 32 : 16);
+    const long long share = (units + nsm - 1) / nsm;
+    int per_sm = 1;
+    while (per_sm < share && per_sm < cap) per_sm *= 2;
+    if (per_sm <= 4) {
+        *NT = 1024;
+        *G = per_sm;
+        return;
+    }
+    auto fit_outages = [&]() {
+        if (!outages || (long long)nv * *G <= 8192) return;
+        *NT = 512;
+        while (*G > 1 && (long long)nv * *G > 8192) *G /= 2;
+    };
+    if (mixed) {
+        const bool mid = per_sm <= 32;
+        *NT = mid && !outages && (long long)nv * per_sm >= 24000 ? 1024 : mid && 4 * share <= 3 * per_sm ? 256 : 512;
+        *G = std::min(gbpf::MAX_SLOTS, per_sm / (1024 / *NT));
+        return fit_outages();
+    }
+    double best = 0.0;
+    *NT = 0;
+    for (int t : {512, 1024, 256})
+        for (int slots = t == 1024 ? 32 : 2; slots <= gbpf::MAX_SLOTS; slots *= 2) {
+            const int on_sm = 1024 / t;  // resident CTAs
+            if (slots * on_sm > cap || slots * on_sm < 8) continue;
+            const long long ctas = (units + slots - 1) / slots, per = (ctas + nsm - 1) / nsm;
+            const bool refill = per > on_sm;
+            if (refill && nv < 400 && slots * on_sm < per_sm) continue;
+            double cost = refill ? (double)units / nsm + slots : per * slots + (outages ? 0.5 * slots : 0.0);
+            cost *= slots == 32 ? 0.84 : slots == 4 ? (outages ? 1.05 : 1.12) : slots == 2 ? 1.25 : 1.0;
+            if (refill && slots * on_sm == 8) cost *= 1.2;
+            if (per == 1 && on_sm > 1) cost *= 1.05;
+            if (!*NT || cost < best) {
+                best = cost;
+                *NT = t;
+                *G = slots;
+            }
+        }
+    if (!*NT) {  // (every candidate is above the cap)
+        *NT = 512;
+        *G = std::max(1, per_sm / 2);
+    }
+    fit_outages();
+}
+
+void choose_shape(const gbpf_solver* s, long long units, bool mixed, int* NT, int* G) {
     const int c = size_class(units);
     if (s->table_NT[c]) {
         *NT = s->table_NT[c];
@@ -314,19 +376,13 @@ void choose_shape(const gbpf_solver* s, long long units, int* NT, int* G) {
         return;
     }
     const int nv = std::max(1, s->plan.nv);
+    if (!s->fixed_NT && !s->fixed_G) return batch_shape(s->nsm, nv, units, mixed, false, NT, G);
     const int cap = nv <= 4096 ? 64 : (nv <= 16384 ? 32 : 16);
     const long long share = (units + s->nsm - 1) / s->nsm;
     int per_sm = 1;
     while (per_sm < share && per_sm < cap) per_sm *= 2;
-    int nt = s->fixed_NT, g = s->fixed_G;
-    if (!nt && !g) {
-        nt = per_sm <= 4 ? 1024 : 512;
-    } else if (!nt) {
-        nt = 512;
-    }
-    if (!g) g = std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / nt)));
-    *NT = nt;
-    *G = g;
+    *NT = s->fixed_NT ? s->fixed_NT : 512;
+    *G = s->fixed_G ? s->fixed_G : std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / *NT)));
 }
 
 // The schedule of one CTA shape: tasks dealt to NT / G workers, uploaded next to the
@@ -514,7 +570,7 @@ int enqueue_launch(gbpf_solver* s, LaunchRes& R, gbpf::Batch& b, long long units
                    int* G_out, int* NT_out) {
     if (units <= 0) return fail(std::string(who) + ": empty batch");
     int NT = 0, G = 0;
-    choose_shape(s, units, &NT, &G);
+    choose_shape(s, units, b.mixed != 0, &NT, &G);
     Shape* sh = nullptr;
     if (int rc = get_shape(s, NT, G, &sh)) return rc;
     const int grid = grid_size(s->nsm, sh->occ, (units + G - 1) / G, b.mixed != 0);
@@ -690,6 +746,8 @@ int job_slots(int Gmax, int nv, int budget) {
 
 }  // namespace
 
+constexpr int DEFAULT_SLOT_BUDGET = 16384;
+
 // A launch context for several topologies at once: its own stream, scratch, control blocks
 // and staging buffers. The topologies (gbpf_solver) keep their plans; a group launch borrows
 // them and must not overlap a call on the same solver.
@@ -700,7 +758,7 @@ struct gbpf_group {
     DBuf scr, bjobs, bctl, btab, bin, bout, bisl;
     gbpf_stats last{};
     int fixed_NT = 0;              // threads per CTA (0: by the group rule)
-    int slot_budget = 16384;       // variable buses x case slots a CTA may hold per job (measured best on the
+    int slot_budget = DEFAULT_SLOT_BUDGET;  // variable buses x case slots a CTA may hold per job (measured best on the
                                    // 256-grid batch: 8,192 +5 %, 32,768 +8 % time)
     ~gbpf_group() {
         for (DBuf* b : {&scr, &bjobs, &bctl, &btab, &bin, &bout, &bisl}) b->release();
@@ -735,9 +793,14 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
         units += J.n_cases;
     }
     int NT = 0, Gmax = 0;
-    group_shape(g->nsm, units, &NT, &Gmax);
-    if (g->fixed_NT) NT = g->fixed_NT;
     const bool mixed = p.precision == 1;
+    group_shape(g->nsm, units, &NT, &Gmax);
+    int alone = 0;  // slots of a launch's only job, by its own batch rule
+    if (nj == 1 && !g->fixed_NT && !jobs[0].cases_per_cta && g->slot_budget == DEFAULT_SLOT_BUDGET) {
+        batch_shape(g->nsm, std::max(1, jobs[0].solver->plan.nv), units, mixed, jobs[0].out_ptr != nullptr, &NT, &alone);
+        Gmax = alone;
+    }
+    if (g->fixed_NT) NT = g->fixed_NT;
     // largest work first, so the long jobs start early and the short ones fill the tail
     std::vector<int> order(nj);
     for (int j = 0; j < nj; ++j) order[j] = j;
@@ -757,7 +820,7 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     // a job whose cases all start from one V0 on the base Ybus without pins gets a shared start
     // (its first evaluation and factorization once, start_kernel)
     auto job_slots_of = [&](const gbpf_job& J) {
-        return J.cases_per_cta ? J.cases_per_cta : job_slots(Gmax, J.solver->plan.nv, g->slot_budget);
+        return J.cases_per_cta ? J.cases_per_cta : alone ? alone : job_slots(Gmax, J.solver->plan.nv, g->slot_budget);
     };
     auto shares = [&](const gbpf_job& J) {
         return p.shared_start && J.n_cases >= SHARE_MIN_CASES && !J.v0_per_col && !J.st_ptr && !J.out_ptr && !J.pin &&
@@ -1003,7 +1066,7 @@ gbpf_solver* gbpf_create_ex(int n, const int32_t* Yp, const int32_t* Yj, const d
     s->Yj.assign(Yj, Yj + nnz);
     s->Yx.assign(Yx, Yx + 2 * (size_t)nnz);
     if (setup(s.get(), cases_per_cta, threads_per_cta)) return nullptr;
-    std::string e = gbpf::build_plan(s->plan, n, Yp, Yj, nnz, pv, npv, pq, npq, 1);
+    std::string e = gbpf::build_plan(s->plan, n, Yp, Yj, nnz, pv, npv, pq, npq, 0);
     if (!e.empty()) {
         fail("gbpf_create: " + e);
         return nullptr;
@@ -1033,7 +1096,7 @@ int gbpf_get_info(gbpf_solver* s, gbpf_info* o) {
     o->n_levels = p.nlev;
     o->n_back_levels = p.nblev;
     int NT = 0, G = 0;  // the shape of a batch that fills the device
-    choose_shape(s, 1LL << 40, &NT, &G);
+    choose_shape(s, 1LL << 40, true, &NT, &G);
     o->cases_per_cta = G;
     o->threads_per_cta = NT;
     o->workers = NT / G;
@@ -1048,8 +1111,8 @@ int gbpf_get_info(gbpf_solver* s, gbpf_info* o) {
 int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta) {
     if (!s) return fail("null solver");
     const int cap = std::max(1, std::min(gbpf::MAX_SLOTS, max_cases_per_cta));
-    for (int NT : {1024, 512})
-        for (int G = 1; G <= (NT == 1024 ? std::min(cap, 4) : cap); G *= 2) {  // 1,024 threads: <= 4 slots
+    for (int NT : {1024, 512, 256})
+        for (int G = NT == 256 ? 2 : 1; G <= (NT == 256 ? std::min(cap, 8) : cap); G *= 2) {  // (batch_shape's)
             Shape* sh = nullptr;
             if (int rc = get_shape(s, NT, G, &sh)) return rc;
         }
@@ -1059,7 +1122,7 @@ int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta) {
 int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta) {
     if (!s || !threads_per_cta || !cases_per_cta) return fail("null argument");
     if (units <= 0) return fail("get_shape: units must be > 0");
-    choose_shape(s, units, threads_per_cta, cases_per_cta);
+    choose_shape(s, units, true, threads_per_cta, cases_per_cta);
     return 0;
 }
 

@@ -135,12 +135,9 @@ void layout(const std::vector<Task>& tasks, int nlev, int nwarps, int wpw, std::
         if (tasks[i].head) by_level[tasks[i].level].push_back(i);
     const int W = nwarps * wpw;
     std::vector<long long> wts, bw;
-    std::vector<int> who, idx;
-    std::vector<std::vector<int>> units;    // task indices; ~i = a recomputing copy of diagonal task i
-    std::vector<std::vector<int>> bundles;  // unit indices
-    using Bundle = std::vector<std::vector<int>>;                // its units' task lists
-    std::vector<std::vector<std::vector<Bundle>>> mine(nwarps);  // [warp][level]
-    for (auto& m : mine) m.resize(nlev);
+    std::vector<int> who, idx, utask, uat, bat, mine;  // units: tasks utask[uat[i] ..) (~q: a recomputing copy of
+                                                       // diagonal task q); bundles: units idx[bat[b] ..)
+    std::vector<std::vector<int>> wout(nwarps), wend(nwarps);  // every warp's steps, and their count after each level
     auto task_of = [](int q) { return q < 0 ? ~q : q; };
     for (int h = 0; h < nlev; ++h) {
         const auto& ids = by_level[h];
@@ -151,95 +148,97 @@ void layout(const std::vector<Task>& tasks, int nlev, int nwarps, int wpw, std::
         // segments (0: never cut)
         const long long cap = chain_cap > 0.0 ? std::max<long long>(1, (long long)std::ceil(chain_cap * (double)total / W))
                                               : std::numeric_limits<long long>::max();
-        units.clear();
+        utask.clear();
+        uat.clear();
         wts.clear();
+        auto open = [&](int q) {
+            uat.push_back((int)utask.size());
+            utask.push_back(q);
+        };
         for (int id : ids) {
             long long cw = 0;
             for (int q = id; q >= 0; q = tasks[q].next) cw += tasks[q].w;
+            open(id);
             if (cw <= cap || tasks[id].next < 0) {
-                units.emplace_back();
-                for (int q = id; q >= 0; q = tasks[q].next) units.back().push_back(q);
+                for (int q = tasks[id].next; q >= 0; q = tasks[q].next) utask.push_back(q);
                 wts.push_back(cw);
                 continue;
             }
             // segments: [diagonal, L...], then [recomputed diagonal, L...] ...
-            units.emplace_back(1, id);
             long long uw = tasks[id].w;
             int nl = 0;
             for (int q = tasks[id].next; q >= 0; q = tasks[q].next) {
                 if (nl > 0 && uw + tasks[q].w > cap) {
                     wts.push_back(uw);
-                    units.emplace_back(1, ~id);
+                    open(~id);
                     uw = tasks[id].w;
                     nl = 0;
                 }
-                units.back().push_back(q);
+                utask.push_back(q);
                 uw += tasks[q].w;
                 ++nl;
             }
             wts.push_back(uw);
         }
-        const int nu = (int)units.size();
-                idx.resize(nu);
+        const int nu = (int)uat.size();
+        uat.push_back((int)utask.size());
+        idx.resize(nu);
         for (int i = 0; i < nu; ++i) idx[i] = i;
-        auto fwd = [&](int i) { return mixed_kinds && (tasks[task_of(units[i][0])].code & 3) == TK_FWD; };
+        auto fwd = [&](int i) { return mixed_kinds && (tasks[task_of(utask[uat[i]])].code & 3) == TK_FWD; };
         std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
             return fwd(a) != fwd(b) ? !fwd(a) : wts[a] > wts[b];
         });
-        bundles.clear();
+        bat.clear();
         bw.clear();
         for (int i = 0; i < nu; ++i) {
-            if (bundles.empty() || (int)bundles.back().size() >= wpw || fwd(bundles.back()[0]) != fwd(idx[i])) {
-                bundles.emplace_back();
+            if (bat.empty() || i - bat.back() >= wpw || fwd(idx[bat.back()]) != fwd(idx[i])) {
+                bat.push_back(i);
                 bw.push_back(0);
             }
-            bundles.back().push_back(idx[i]);
             bw.back() = std::max(bw.back(), wts[idx[i]]);
         }
+        const int nb = (int)bat.size();
+        bat.push_back(nu);
         const int mx = deal(bw, nwarps, who);
         if (level_work) (*level_work)[h] += mx;
-        for (size_t b = 0; b < bundles.size(); ++b) {
-            auto& dst = mine[who[b]][h];
-            dst.emplace_back();
-            for (int u : bundles[b]) dst.back().push_back(units[u]);
-        }
         // within a warp, bundles in the order of their key (the factor position they work on):
         // at any moment the warps of a CTA are at similar positions and share the blocks they
         // read in cache
-        for (auto& m : mine)
-            std::stable_sort(m[h].begin(), m[h].end(), [&](const auto& a, const auto& b) {
-                return key[task_of(a[0][0])] < key[task_of(b[0][0])];
-            });
+        mine.resize(nb);
+        for (int b = 0; b < nb; ++b) mine[b] = b;
+        auto bkey = [&](int b) { return key[task_of(utask[uat[idx[bat[b]]]])]; };
+        std::stable_sort(mine.begin(), mine.end(), [&](int a, int b) {
+            return who[a] != who[b] ? who[a] < who[b] : bkey(a) < bkey(b);
+        });
+        for (int b : mine) {
+            std::vector<int>& o = wout[who[b]];
+            int len = 0;
+            for (int i = bat[b]; i < bat[b + 1]; ++i) len = std::max(len, uat[idx[i] + 1] - uat[idx[i]]);
+            for (int k = 0; k < len; ++k)
+                for (int w = 0; w < wpw; ++w) {
+                    const int i = bat[b] + w;
+                    const int at = i < bat[b + 1] ? uat[idx[i]] + k : -1;
+                    if (at < 0 || at >= uat[idx[i] + 1]) {
+                        o.insert(o.end(), {-1, 0, 0, 0});
+                        continue;
+                    }
+                    const Task& t = tasks[task_of(utask[at])];
+                    o.insert(o.end(), {t.dst, utask[at] < 0 ? (t.code | TASK_NOSTORE) : t.code, t.p0, t.p1});
+                }
+        }
+        for (int u = 0; u < nwarps; ++u) wend[u].push_back((int)(wout[u].size() / (4 * (size_t)wpw)));
     }
     out.clear();
     ptr.clear();
-    const int null_task[4] = {-1, 0, 0, 0};
     int steps = 0;
     for (int u = 0; u < nwarps; ++u) {
-        for (int h = 0; h < nlev; ++h) {
-            ptr.push_back(steps);
-            for (const auto& bundle : mine[u][h]) {
-                size_t len = 0;
-                for (const auto& unit : bundle) len = std::max(len, unit.size());
-                for (size_t k = 0; k < len; ++k, ++steps)
-                    for (int w = 0; w < wpw; ++w) {
-                        if (w >= (int)bundle.size() || k >= bundle[w].size()) {
-                            out.insert(out.end(), null_task, null_task + 4);
-                            continue;
-                        }
-                        const int q = bundle[w][k];
-                        const Task& t = tasks[task_of(q)];
-                        out.push_back(t.dst);
-                        out.push_back(q < 0 ? (t.code | TASK_NOSTORE) : t.code);
-                        out.push_back(t.p0);
-                        out.push_back(t.p1);
-                    }
-            }
-        }
         ptr.push_back(steps);
+        for (int e : wend[u]) ptr.push_back(steps + e);
+        steps = ptr.back();
+        out.insert(out.end(), wout[u].begin(), wout[u].end());
     }
     // read ahead by the kernel: a step past the last, a range past the last level
-    for (int w = 0; w < wpw; ++w) out.insert(out.end(), null_task, null_task + 4);
+    for (int w = 0; w < wpw; ++w) out.insert(out.end(), {-1, 0, 0, 0});
     ptr.push_back(steps);
 }
 
@@ -408,7 +407,7 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
     }
 
     // tasks
-    const int W = p.W = std::max(1, workers);
+    const int W = p.W = workers;
     std::vector<Task> A, C;
     p.pairs.clear();
     p.pair_level.clear();
@@ -471,17 +470,19 @@ std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, co
     if (p.pairs.size() / 2 >= (size_t)1 << 31) return "too many pairs";
     p.tasksA = std::move(A);
     p.tasksC = std::move(C);
-    p.warp = std::min(32, std::max(1, W / 16));
-    while (W % p.warp) --p.warp;
-    Schedule sc;
-    make_schedule(p, W / p.warp, p.warp, sc, chain_cap);
-    p.taskA = std::move(sc.taskA);
-    p.ptrA = std::move(sc.ptrA);
-    p.taskF = std::move(sc.taskF);
-    p.ptrF = std::move(sc.ptrF);
-    p.taskC = std::move(sc.taskC);
-    p.ptrC = std::move(sc.ptrC);
-    p.level_work = std::move(sc.level_work);
+    if (W > 0) {
+        p.warp = std::min(32, std::max(1, W / 16));
+        while (W % p.warp) --p.warp;
+        Schedule sc;
+        make_schedule(p, W / p.warp, p.warp, sc, chain_cap);
+        p.taskA = std::move(sc.taskA);
+        p.ptrA = std::move(sc.ptrA);
+        p.taskF = std::move(sc.taskF);
+        p.ptrF = std::move(sc.ptrF);
+        p.taskC = std::move(sc.taskC);
+        p.ptrC = std::move(sc.ptrC);
+        p.level_work = std::move(sc.level_work);
+    }
     return std::string();
 }
 
@@ -664,48 +665,42 @@ static inline void mm_sub(double* acc, const double* a, const double* b) {
 bool host_factor(const Plan& p, double* blk, double* pmin, double* pmax) {
     double mn = INFINITY, mx = 0.0;
     bool ok = true;
-    for (int h = 0; h < p.nlev; ++h) {
-        for (int w = 0; w < p.W; ++w) {
-            double dinv[4] = {0, 0, 0, 0};  // the worker's last inverse diagonal block
-            for (int t = first_step(p, p.ptrA, p.nlev, h, w); t < last_step(p, p.ptrA, p.nlev, h, w); ++t) {
-                const int* T = &p.taskA[4 * ((size_t)t * p.warp + w % p.warp)];
-                const int kind = T[1] & 3;
-                if (kind == TK_FWD || T[0] < 0) continue;
-                double acc[4] = {0, 0, 0, 0};
-                if (!(T[1] & TASK_FILL))
-                    for (int e = 0; e < 4; ++e) acc[e] = blk[4 * (size_t)T[0] + e];
-                for (int q = T[2]; q < T[3]; ++q)
-                    mm_sub(acc, blk + 4 * (size_t)p.pairs[2 * q], blk + 4 * (size_t)p.pairs[2 * q + 1]);
-                double* o = blk + 4 * (size_t)T[0];
-                if (kind == TK_DIAG) {
-                    const int row = T[1] >> TASK_ROW_SHIFT;
-                    const double det = acc[0] * acc[3] - acc[1] * acc[2];
-                    const double inv = 1.0 / det;
-                    dinv[0] = acc[3] * inv;
-                    dinv[1] = -acc[1] * inv;
-                    dinv[2] = -acc[2] * inv;
-                    dinv[3] = acc[0] * inv;
-                    if (T[1] & TASK_NOSTORE) continue;  // a segment's copy: the inverse stays in dinv
-                    const double u0 = std::fabs(acc[0]);
-                    const double u1 = std::fabs(det / acc[0]);
-                    if (!(u0 > 0.0) || !std::isfinite(u0) || !std::isfinite(det)) ok = false;
-                    mn = std::min(mn, u0);
-                    mx = std::max(mx, u0);
-                    if (p.row_pq[row]) {
-                        if (!(u1 > 0.0) || !std::isfinite(u1)) ok = false;
-                        mn = std::min(mn, u1);
-                        mx = std::max(mx, u1);
-                    }
-                    for (int e = 0; e < 4; ++e) blk[4 * ((size_t)p.nblk + row) + e] = dinv[e];
-                } else if (T[1] & TASK_SCALE) {
-                    o[0] = acc[0] * dinv[0] + acc[1] * dinv[2];
-                    o[1] = acc[0] * dinv[1] + acc[1] * dinv[3];
-                    o[2] = acc[2] * dinv[0] + acc[3] * dinv[2];
-                    o[3] = acc[2] * dinv[1] + acc[3] * dinv[3];
-                } else {
-                    for (int e = 0; e < 4; ++e) o[e] = acc[e];
-                }
+    double dinv[4] = {0, 0, 0, 0};  // the last inverse diagonal block
+    for (const Task& t : p.tasksA) {  // in pivot order: what a task reads is final
+        const int kind = t.code & 3;
+        if (kind == TK_FWD) continue;
+        double acc[4] = {0, 0, 0, 0};
+        if (!(t.code & TASK_FILL))
+            for (int e = 0; e < 4; ++e) acc[e] = blk[4 * (size_t)t.dst + e];
+        for (int q = t.p0; q < t.p1; ++q)
+            mm_sub(acc, blk + 4 * (size_t)p.pairs[2 * q], blk + 4 * (size_t)p.pairs[2 * q + 1]);
+        double* o = blk + 4 * (size_t)t.dst;
+        if (kind == TK_DIAG) {
+            const int row = t.code >> TASK_ROW_SHIFT;
+            const double det = acc[0] * acc[3] - acc[1] * acc[2];
+            const double inv = 1.0 / det;
+            dinv[0] = acc[3] * inv;
+            dinv[1] = -acc[1] * inv;
+            dinv[2] = -acc[2] * inv;
+            dinv[3] = acc[0] * inv;
+            const double u0 = std::fabs(acc[0]);
+            const double u1 = std::fabs(det / acc[0]);
+            if (!(u0 > 0.0) || !std::isfinite(u0) || !std::isfinite(det)) ok = false;
+            mn = std::min(mn, u0);
+            mx = std::max(mx, u0);
+            if (p.row_pq[row]) {
+                if (!(u1 > 0.0) || !std::isfinite(u1)) ok = false;
+                mn = std::min(mn, u1);
+                mx = std::max(mx, u1);
             }
+            for (int e = 0; e < 4; ++e) blk[4 * ((size_t)p.nblk + row) + e] = dinv[e];
+        } else if (t.code & TASK_SCALE) {
+            o[0] = acc[0] * dinv[0] + acc[1] * dinv[2];
+            o[1] = acc[0] * dinv[1] + acc[1] * dinv[3];
+            o[2] = acc[2] * dinv[0] + acc[3] * dinv[2];
+            o[3] = acc[2] * dinv[1] + acc[3] * dinv[3];
+        } else {
+            for (int e = 0; e < 4; ++e) o[e] = acc[e];
         }
     }
     *pmin = mn;

@@ -102,7 +102,8 @@ struct Plan {
     std::vector<int> level_work;    // per level: max worker load (critical path estimate)
 };
 
-// Build everything topology-only. Returns an empty string on success, else the error.
+// Build everything topology-only, with a schedule for `workers` workers in the plan itself (0: none).
+// Returns an empty string on success, else the error.
 std::string build_plan(Plan& p, int n, const int* Yp, const int* Yj, int nnz, const int* pv, int npv,
                        const int* pq, int npq, int workers, double chain_cap = 1.0);
 
