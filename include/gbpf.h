@@ -48,8 +48,9 @@ typedef struct gbpf_params {
     int shared_start;    /* 1: a batch of at least 16 cases that all start from one V0 on the base
                             Ybus without pins evaluates and factors that start once (a one-CTA
                             prologue) and every case's first step solves with it -- for bulk
-                            batches; 0: every case evaluates and factors its own start (no
-                            prologue on the launch's critical path: latency-bound serving) */
+                            batches; 2: where that is the faster way (the same results either way);
+                            0: every case evaluates and factors its own start (no prologue on the
+                            launch's critical path: latency-bound serving) */
     int phase_timers;    /* 1: the Newton kernel sums SM clock cycles per phase over its CTAs into
                             gbpf_stats.phase_cycles (single-topology launches; 0: off, the default) */
     int eager_jacobian;  /* mixed, vote_rule 1: 0 (default) leaves the float Jacobian out of an

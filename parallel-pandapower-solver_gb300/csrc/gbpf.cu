@@ -554,8 +554,16 @@ int check_params(const gbpf_params& p, const char* who) {
     return 0;
 }
 
-// A shared start pays for its one-CTA prologue only over enough cases starting from it.
+// A shared start (gbpf_params.shared_start 1) is taken from this many cases on; with 2 (where it
+// pays) only where its one-CTA prologue, which every case waits for, costs less than what the
+// cases of one SM save by it. Buses x cases an SM, measured over 118 to 20,000 buses and 16 to
+// 4,864 cases: the line lies near 12,000 mixed and 5,000 double (2,000 buses mixed: 96 cases 0.98
+// ms with the prologue, 0.88 without, 1,216 cases 2.36 and 2.41; double 1.41 and 1.24, 3.97 and
+// 4.34), and with one case an SM it never pays.
 constexpr long long SHARE_MIN_CASES = 16;
+bool start_pays(int nsm, long long cases, long long bus_cases, bool mixed) {
+    return cases > nsm && bus_cases >= (mixed ? 12000LL : 5000LL) * nsm;
+}
 
 // The launch of `units` work items (cases, or lanes) enqueued on a stream with its own
 // scratch and control block; read back with finish_launch.
@@ -593,7 +601,8 @@ int enqueue_launch(gbpf_solver* s, LaunchRes& R, gbpf::Batch& b, long long units
     b.err = reinterpret_cast<int*>(ctl + 24);
     // shared start: every case from the same V0 on the base Ybus without pins -- its first
     // evaluation and factorization are computed once (start_kernel) for the whole launch
-    const bool share = b.share_ok && units >= SHARE_MIN_CASES && b.v0_shared && b.ymode == 0 && !b.pin && !b.ref_bus &&
+    const bool share = b.share_ok && units >= SHARE_MIN_CASES &&
+                       (b.share_ok != 2 || start_pays(s->nsm, units, units * s->n, b.mixed != 0)) && b.v0_shared && b.ymode == 0 && !b.pin && !b.ref_bus &&
                        (!b.mixed || b.vote_rule == 1);
     gbpf::StartJob sj{};
     const size_t tab_bytes = ((size_t)s->n * 64 + 255) & ~(size_t)255;
@@ -717,7 +726,7 @@ void fill_common(gbpf::Batch& b, const gbpf_solver* s, const gbpf_params& p) {
     // step like nr_klu)
     b.chord_tol = b.mixed && b.vote_rule == 1 && p.chord_tol > 0.0 ? p.chord_tol : 0.0;
     b.lazy_jac = b.chord_tol > 0.0 && !p.eager_jacobian;
-    b.share_ok = p.shared_start != 0;
+    b.share_ok = p.shared_start;
     b.timers = p.phase_timers != 0;
     b.check_v0 = p.check_v0;
     b.rcond_min64 = p.pivot_ratio_double * s->plan.rcond0;  // nr_klu.cpp:567 REUSE_RCOND_RATIO = 1e-3
@@ -822,8 +831,11 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     auto job_slots_of = [&](const gbpf_job& J) {
         return J.cases_per_cta ? J.cases_per_cta : alone ? alone : job_slots(Gmax, J.solver->plan.nv, g->slot_budget);
     };
+    long long bus_cases = 0;
+    for (int j = 0; j < nj; ++j) bus_cases += (long long)jobs[j].n_cases * jobs[j].solver->n;
+    const bool starts = p.shared_start == 1 || (p.shared_start == 2 && start_pays(g->nsm, units, bus_cases, mixed));
     auto shares = [&](const gbpf_job& J) {
-        return p.shared_start && J.n_cases >= SHARE_MIN_CASES && !J.v0_per_col && !J.st_ptr && !J.out_ptr && !J.pin &&
+        return starts && J.n_cases >= SHARE_MIN_CASES && !J.v0_per_col && !J.st_ptr && !J.out_ptr && !J.pin &&
                (!mixed || p.vote_rule == 1);
     };
     for (int j = 0; j < nj; ++j) {

@@ -989,11 +989,12 @@ struct Quad {
 // through the levels and back. Pivot statistics per slot go to smin / smax (as ordered bits).
 // With `solo` a slot index, P is the one-slot schedule and all threads work on that slot. Slots
 // flagged in `chord` keep the factors already in `fac` and run the substitutions only. QUADS: a
-// double pass takes the plan's quad levels (DevPlan::quad_from, quad_to). Float passes take none:
+// double pass takes the plan's quad levels (DevPlan::quad_from, quad_to); BACK: with the backward
+// substitution (the shared start's pass is there for its factors). Float passes take none:
 // they wait for memory rather than for a chain of instructions, and one lane a task has more
 // tasks in flight (one case of the 2,000-bus grid: factor levels 0.43 ms, 0.54 with quads
 // throughout, 0.50 with quads in the narrow levels only).
-template <typename real, bool TIMED = false, bool QUADS = true>
+template <typename real, bool TIMED = false, bool QUADS = true, bool BACK = true>
 __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const double2* R, typename V4<real>::t2* y,
                         const int* on, int lg, unsigned long long* smin, unsigned long long* smax, const int* chord,
                         bool factor_any, typename V4<real>::t* dinv_smem, int solo = -1, unsigned long long* ph = nullptr,
@@ -1011,12 +1012,12 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
         lane_forward<real>(P, L, fac, R, y, dinv_smem, pv, 0, hq);
         if (hq < P.nlev) Quad<real>(P, L, fac, y).forward(R, pv, hq, P.nlev);
         if constexpr (TIMED) phase_mark(ph, clk, 1);
-        if (P.quad_to) Quad<real>(P, L, fac, y).backward(0, P.quad_to);
-        lane_backward<real>(P, L, fac, y, P.quad_to, P.nblev);
+        if (BACK && P.quad_to) Quad<real>(P, L, fac, y).backward(0, P.quad_to);
+        if (BACK) lane_backward<real>(P, L, fac, y, P.quad_to, P.nblev);
     } else {
         lane_forward<real>(P, L, fac, R, y, dinv_smem, pv, 0, P.nlev);
         if constexpr (TIMED) phase_mark(ph, clk, 1);
-        lane_backward<real>(P, L, fac, y, 0, P.nblev);
+        if (BACK) lane_backward<real>(P, L, fac, y, 0, P.nblev);
     }
     if (L.act) {
         lower_min(&smin[L.s], pv.lo_bits());
@@ -2040,10 +2041,11 @@ __global__ void __launch_bounds__(NTB, 1) start_kernel(const StartJob* jobs) {
     }
     __syncthreads();
     if (sj.mixed)
-        lu_pass<float>(P, reinterpret_cast<float4*>(sj.fac1), sj.R0, reinterpret_cast<float2*>(sj.y0), s_on, 0, s_min,
-                       s_max, nullptr, true, nullptr);
+        lu_pass<float, false, true, false>(P, reinterpret_cast<float4*>(sj.fac1), sj.R0, reinterpret_cast<float2*>(sj.y0),
+                                           s_on, 0, s_min, s_max, nullptr, true, nullptr);
     else
-        lu_pass<double>(P, reinterpret_cast<double4_32a*>(sj.fac1), sj.R0, sj.y0, s_on, 0, s_min, s_max, nullptr, true, nullptr);
+        lu_pass<double, false, true, false>(P, reinterpret_cast<double4_32a*>(sj.fac1), sj.R0, sj.y0, s_on, 0, s_min, s_max,
+                                            nullptr, true, nullptr);
     if (tid == 0) *sj.ok0 = pivots_ok(s_min[0], s_max[0], sj.rcond_min) ? 1 : 0;
 }
 

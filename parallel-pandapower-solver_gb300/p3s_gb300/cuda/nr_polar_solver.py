@@ -62,7 +62,7 @@ class PolarNewtonSolverCUDA:
     def _params(self, max_iter, tol):
         return GpuSolver.params(max_iter, tol, self.line_search, self.precision, self.mixed_switch,
                                 pivot_ratio_double=self._rcond_ratio, pivot_ratio_single=self._rcond_ratio_single,
-                                vote_rule=self.vote_rule, polish=self.polish, vtol=self.vtol)
+                                vote_rule=self.vote_rule, polish=self.polish, vtol=self.vtol, shared_start="auto")
 
     def _record(self, B, r, st=None):
         own = st is None  # a launch of this solver (not of a group): its cases' mismatch is recorded

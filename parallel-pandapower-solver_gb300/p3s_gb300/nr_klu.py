@@ -78,7 +78,7 @@ class Solver:
                 raise _err("solve_batch: V0 (n,T) shape mismatch")
         elif V0.shape[0] != self.n:
             raise _err("solve_batch: V0 (n,) length mismatch")
-        p = GpuSolver.params(max_iter, tol, line_search, check_v0=True)
+        p = GpuSolver.params(max_iter, tol, line_search, check_v0=True, shared_start="auto")
         return self._s.solve_batch(Sbus, V0, p)
 
     def solve_batch_contingency(self, Yx_mag, Yx_ang, Sbus, V0, pin, max_iter: int = 30, tol: float = 1e-8,

@@ -33,3 +33,23 @@ def test_small_shapes_agree_bit_for_bit(n):
         if precision == "double":
             assert np.array_equal(first["iterations"], ref["iterations"])
             assert np.abs(first["V"] - ref["V"]).max() < 1e-11
+
+
+@pytest.mark.parametrize("cases", [15, 16, 153, 3200])
+def test_shared_start_where_it_pays_changes_no_result(cases):
+    """Below 16 cases never, then only where the prologue pays (3,200 cases of 257 buses: double yes, mixed
+    no): the same bits as always and never sharing the start."""
+    g = make_grid(257, seed=257, max_drop_pu=0.05)
+    S = scenario_injections(g, cases, seed=3)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    for precision in ("double", "mixed"):
+        r, first = {}, {}
+        for how in (True, False, "auto"):
+            r[how] = s.solve_batch(S, g.V0, GpuSolver.params(precision=precision, shared_start=how))
+            first[how] = s.stats["first_steps"]
+        assert first[True] == (cases if cases >= 16 else 0) and first[False] == 0
+        assert first["auto"] == (cases if cases == 3200 and precision == "double" else 0)
+        for how in (False, "auto"):
+            assert np.array_equal(r[how]["V"], r[True]["V"])
+            assert np.array_equal(r[how]["iterations"], r[True]["iterations"])
+        assert r[True]["converged"].all()
