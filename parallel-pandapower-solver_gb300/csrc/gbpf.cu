@@ -75,6 +75,27 @@ struct DBuf {
     }
 };
 
+// Page-locked block for a call's small results. A copy from the device to pageable memory holds
+// the caller until it has arrived, ~8 us each after the kernel: into this block several copies
+// queue up behind the launch and one synchronisation waits for all. Up to STAGE_MAX bytes; larger
+// results go to the caller's memory directly, where the transfer itself is what counts.
+constexpr size_t STAGE_MAX = 256u << 10;
+
+struct HStage {
+    char* p = nullptr;
+    char* get(size_t b) {  // null: use the caller's memory
+        if (b > STAGE_MAX) return nullptr;
+        if (!p && cudaMallocHost(&p, STAGE_MAX) != cudaSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+        }
+        return p;
+    }
+    ~HStage() {
+        if (p) cudaFreeHost(p);
+    }
+};
+
 template <typename T>
 cudaError_t upload(DBuf& b, const std::vector<T>& v) {
     cudaError_t e = b.ensure(v.size() * sizeof(T));
@@ -133,6 +154,7 @@ struct Shape {
     }
 };
 
+constexpr size_t DC_KEEP = 64u << 20;  // a DC start's work arrays beyond this are freed after the call
 constexpr int N_SIZE_CLASSES = 48;  // batch sizes by ceil(log2(work items))
 
 // Resources of one launch in flight: stream, events, scratch and buffers. The solver's own
@@ -176,6 +198,8 @@ struct gbpf_solver {
     DBuf scr;
     // per-call buffers (grow-only)
     DBuf bS, bV0, bV, bit, bcv, bctl, blane, bstp, bstk, bstv, bYd, bpin, btab, bjobs;
+    HStage hstage;        // small results of synchronous calls
+    DBuf bdc;             // work arrays of the DC start (kept up to DC_KEEP bytes)
     DBuf bmis;            // final mismatch of every case of the last synchronous call
     long long mis_n = 0;  // its case count (0: none recorded)
     // islanding buffers (grow-only)
@@ -195,7 +219,7 @@ struct gbpf_solver {
         shapes.clear();
         for (DBuf* b : {&dYp, &dYj, &dY, &dY32, &dposmap, &drow_of_bus, &dbus_pq, &dpairs, &drow_pq, &dbus_of_row, &drows, &drows_by_len,
                         &ddpos, &scr, &bS, &bV0, &bV, &bit, &bcv, &bctl, &blane, &bstp, &bstk, &bstv, &bYd, &bpin,
-                        &btab, &bjobs, &bmis, &iin, &iscr, &ibest, &iout, &dbr_f, &dbr_t, &dbr_live, &dbr_pos, &dbr_val,
+                        &btab, &bjobs, &bmis, &bdc, &iin, &iscr, &ibest, &iout, &dbr_f, &dbr_t, &dbr_live, &dbr_pos, &dbr_val,
                         &dslack, &dprio, &dg_ptr, &dg_src, &dshunt})
             b->release();
         for (cudaEvent_t e : {e0, e1, c0, c1})
@@ -765,6 +789,7 @@ struct gbpf_group {
     cudaStream_t stream = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr, c0 = nullptr, c1 = nullptr;
     DBuf scr, bjobs, bctl, btab, bin, bout, bisl;
+    HStage hstage;  // iterations and flags of gbpf_group_solve
     gbpf_stats last{};
     int fixed_NT = 0;              // threads per CTA (0: by the group rule)
     int slot_budget = DEFAULT_SLOT_BUDGET;  // variable buses x case slots a CTA may hold per job (measured best on the
@@ -1238,11 +1263,20 @@ int gbpf_solve_batch(gbpf_solver* s, int T, const double* S, int s_per_col, cons
     if (int rc = gbpf_solve_batch_device(s, T, s->bS.as<double>(), s_per_col, s->bV0.as<double>(), v0_per_col, pp,
                                          s->bV.as<double>(), s->bit.as<int32_t>(), s->bcv.as<uint8_t>()))
         return rc;
-    CK(cudaMemcpyAsync(V, s->bV.p, ob, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaMemcpyAsync(it, s->bit.p, (size_t)T * 4, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaMemcpyAsync(cv, s->bcv.p, (size_t)T, cudaMemcpyDeviceToHost, s->stream));
+    // iterations and flags through the page-locked block, V too where it fits
+    const size_t nit = (size_t)T * 4, small = nit + T;
+    char* hv = s->hstage.get(ob + small);
+    char* hs = hv ? hv + ob : s->hstage.get(small);
+    CK(cudaMemcpyAsync(hs ? (void*)hs : it, s->bit.p, nit, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(hs ? (void*)(hs + nit) : cv, s->bcv.p, (size_t)T, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(hv ? (void*)hv : V, s->bV.p, ob, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaEventRecord(s->c1, s->stream));
     CK(cudaStreamSynchronize(s->stream));
+    if (hs) {
+        std::memcpy(it, hs, nit);
+        std::memcpy(cv, hs + nit, (size_t)T);
+    }
+    if (hv) std::memcpy(V, hv, ob);
     return record_call(s);
 }
 
@@ -1462,40 +1496,47 @@ int gbpf_dc_start_batch(gbpf_solver* s, int T, const double* Pinj, const double*
     std::vector<double> th(n * (size_t)T);
     std::vector<double> th0(n);
     for (size_t i = 0; i < n; ++i) th0[i] = std::atan2(V0[2 * i + 1], V0[2 * i]);
-    DBuf dP, dth, dfac, dR, dy, dout, dpiv, dB, dst, dsh;
-    auto cleanup = [&]() {
-        for (DBuf* b : {&dP, &dth, &dfac, &dR, &dy, &dout, &dpiv, &dB, &dst, &dsh}) b->release();
-    };
+    // one buffer for all work arrays, kept with the solver while it is small: eight to ten
+    // allocations and frees (each free waits for the device) were half of a call's 0.31 ms
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t bP = up(n * 8 * T), bth = up(n * 8), bfac = up((nb + nv) * 32), bR = up(nv * 16 * grid),
+                 bst = dc_stamps ? up(64 * (size_t)s->m) : 0, bsh = dc_stamps ? up(16 * n) : 0,
+                 bB = dc_stamps ? up(16 * nnz) : 0;
+    CK(s->bdc.ensure(2 * bP + bth + bfac + 2 * bR + 256 + bst + bsh + bB));
     struct Guard {
-        std::function<void()> f;
-        ~Guard() { f(); }
-    } guard{cleanup};
+        DBuf& b;
+        ~Guard() {
+            if (b.bytes > DC_KEEP) b.release();
+        }
+    } guard{s->bdc};
+    char* at = s->bdc.as<char>();
+    auto take = [&](size_t b) {
+        char* p = at;
+        at += b;
+        return p;
+    };
+    char *dP = take(bP), *dout = take(bP), *dth = take(bth), *dfac = take(bfac), *dR = take(bR), *dy = take(bR),
+         *dpiv = take(256);
     const double2* Bx = nullptr;
     if (dc_stamps) {  // the DC stamps summed onto the Ybus pattern like the AC ones (COO order)
         if (int rc = ensure_gather(s)) return rc;
-        CK(dst.ensure(64 * (size_t)s->m));
-        CK(dsh.ensure(16 * n));
-        CK(dB.ensure(16 * nnz));
-        CK(cudaMemcpyAsync(dst.p, dc_stamps, 64 * (size_t)s->m, cudaMemcpyHostToDevice, s->stream));
-        CK(cudaMemsetAsync(dsh.p, 0, 16 * n, s->stream));
-        CK(gbpf::launch_ybus_gather((int)nnz, 4 * s->m, s->dg_ptr.as<int>(), s->dg_src.as<int>(), dst.as<double2>(),
-                                    dsh.as<double2>(), dB.as<double2>(), nullptr, s->stream));
-        Bx = dB.as<double2>();
+        char *dst = take(bst), *dsh = take(bsh), *dB = take(bB);
+        CK(cudaMemcpyAsync(dst, dc_stamps, 64 * (size_t)s->m, cudaMemcpyHostToDevice, s->stream));
+        CK(cudaMemsetAsync(dsh, 0, 16 * n, s->stream));
+        CK(gbpf::launch_ybus_gather((int)nnz, 4 * s->m, s->dg_ptr.as<int>(), s->dg_src.as<int>(),
+                                    reinterpret_cast<double2*>(dst), reinterpret_cast<double2*>(dsh),
+                                    reinterpret_cast<double2*>(dB), nullptr, s->stream));
+        Bx = reinterpret_cast<const double2*>(dB);
     }
-    CK(dP.ensure(n * 8 * T));
-    CK(dth.ensure(n * 8));
-    CK(dfac.ensure((nb + nv) * 32));
-    CK(dR.ensure(nv * 16 * grid));
-    CK(dy.ensure(nv * 16 * grid));
-    CK(dout.ensure(n * 8 * T));
-    CK(dpiv.ensure(16));
-    CK(cudaMemcpyAsync(dP.p, Pinj, n * 8 * T, cudaMemcpyHostToDevice, s->stream));
-    CK(cudaMemcpyAsync(dth.p, th0.data(), n * 8, cudaMemcpyHostToDevice, s->stream));
-    CK(gbpf::launch_dc(sh->dp, Bx, dP.as<double>(), T, dth.as<double>(), dfac.as<double4_32a>(), dR.as<double2>(),
-                       dy.as<double2>(), dout.as<double>(), dpiv.as<unsigned long long>(), grid, s->stream));
+    CK(cudaMemcpyAsync(dP, Pinj, n * 8 * T, cudaMemcpyHostToDevice, s->stream));
+    CK(cudaMemcpyAsync(dth, th0.data(), n * 8, cudaMemcpyHostToDevice, s->stream));
+    CK(gbpf::launch_dc(sh->dp, Bx, reinterpret_cast<double*>(dP), T, reinterpret_cast<double*>(dth),
+                       reinterpret_cast<double4_32a*>(dfac), reinterpret_cast<double2*>(dR),
+                       reinterpret_cast<double2*>(dy), reinterpret_cast<double*>(dout),
+                       reinterpret_cast<unsigned long long*>(dpiv), grid, s->stream));
     unsigned long long piv[2];
-    CK(cudaMemcpyAsync(th.data(), dout.p, n * 8 * T, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaMemcpyAsync(piv, dpiv.p, 16, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(th.data(), dout, n * 8 * T, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(piv, dpiv, 16, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     // a zero or non-finite pivot (a DC island without a reference) or non-finite angles:
     // the case keeps the flat start (timeseries.py:244-247)
@@ -1803,8 +1844,8 @@ int gbpf_group_solve(gbpf_group* g, int njobs, const gbpf_job* jobs, const gbpf_
     if (int rc = check_params(p, "group_solve")) return rc;
     // stage every job's inputs in one device buffer and its outputs in another
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    std::vector<size_t> in_at(njobs), out_at(njobs);
-    size_t in_bytes = 0, out_bytes = 0;
+    std::vector<size_t> in_at(njobs), out_at(njobs), small_at(njobs);
+    size_t in_bytes = 0, out_bytes = 0, small_bytes = 0;
     for (int j = 0; j < njobs; ++j) {
         const gbpf_job& J = jobs[j];
         if (!J.solver || J.n_cases <= 0) return fail("group_solve: job " + std::to_string(j) + " is empty");
@@ -1835,10 +1876,14 @@ int gbpf_group_solve(gbpf_group* g, int njobs, const gbpf_job* jobs, const gbpf_
             in_bytes += up((T + 1) * 4) + up((size_t)std::max(J.out_ptr[T], 1) * 4);
         }
         out_at[j] = out_bytes;
-        out_bytes += up(n * T * 16) + up(T * 4) + up(T) + (J.served ? up(n * T) : 0);
+        out_bytes += up(n * T * 16) + (J.served ? up(n * T) : 0);
+        small_at[j] = small_bytes;
+        small_bytes += up(T * 4) + up(T);
     }
+    // the iterations and flags of all jobs lie together behind the voltages
+    const size_t small0 = out_bytes;
     CK(g->bin.ensure(in_bytes));
-    CK(g->bout.ensure(out_bytes));
+    CK(g->bout.ensure(out_bytes + small_bytes));
     CK(cudaEventRecord(g->c0, g->stream));
     std::vector<gbpf_job> dj(jobs, jobs + njobs);
     for (int j = 0; j < njobs; ++j) {
@@ -1875,21 +1920,30 @@ int gbpf_group_solve(gbpf_group* g, int njobs, const gbpf_job* jobs, const gbpf_
         }
         char* o = g->bout.as<char>() + out_at[j];
         D.V = reinterpret_cast<double*>(o);
-        D.iterations = reinterpret_cast<int32_t*>(o + up(n * T * 16));
-        D.converged = reinterpret_cast<uint8_t*>(o + up(n * T * 16) + up(T * 4));
-        if (J.served) D.served = reinterpret_cast<uint8_t*>(o + up(n * T * 16) + up(T * 4) + up(T));
+        if (J.served) D.served = reinterpret_cast<uint8_t*>(o + up(n * T * 16));
+        o = g->bout.as<char>() + small0 + small_at[j];
+        D.iterations = reinterpret_cast<int32_t*>(o);
+        D.converged = reinterpret_cast<uint8_t*>(o + up(T * 4));
     }
     if (int rc = group_run(g, njobs, dj.data(), p, "group_solve")) return rc;
+    char* hs = g->hstage.get(small_bytes);
+    if (hs) CK(cudaMemcpyAsync(hs, g->bout.as<char>() + small0, small_bytes, cudaMemcpyDeviceToHost, g->stream));
     for (int j = 0; j < njobs; ++j) {
         const gbpf_job& J = jobs[j];
         const size_t n = J.solver->n, T = J.n_cases;
         CK(cudaMemcpyAsync(J.V, dj[j].V, n * T * 16, cudaMemcpyDeviceToHost, g->stream));
+        if (J.served) CK(cudaMemcpyAsync(J.served, dj[j].served, n * T, cudaMemcpyDeviceToHost, g->stream));
+        if (hs) continue;
         CK(cudaMemcpyAsync(J.iterations, dj[j].iterations, T * 4, cudaMemcpyDeviceToHost, g->stream));
         CK(cudaMemcpyAsync(J.converged, dj[j].converged, T, cudaMemcpyDeviceToHost, g->stream));
-        if (J.served) CK(cudaMemcpyAsync(J.served, dj[j].served, n * T, cudaMemcpyDeviceToHost, g->stream));
     }
     CK(cudaEventRecord(g->c1, g->stream));
     CK(cudaStreamSynchronize(g->stream));
+    for (int j = 0; hs && j < njobs; ++j) {
+        const size_t T = jobs[j].n_cases;
+        std::memcpy(jobs[j].iterations, hs + small_at[j], T * 4);
+        std::memcpy(jobs[j].converged, hs + small_at[j] + up(T * 4), T);
+    }
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, g->c0, g->c1));
     g->last.call_ms = ms;

@@ -119,6 +119,16 @@ def _start_voltage(grid, init: str, solver: GpuSolver, dc_stamps=None, p_shift=N
     return V
 
 
+def _all_finite(a: np.ndarray) -> bool:
+    """No NaN and no infinity in a complex128 array. A NaN or an infinity makes the sum of the
+    parts non-finite, so a finite sum settles it in one pass without a temporary; only a sum
+    that is not (it may have overflowed) needs the element-wise test."""
+    x = np.ascontiguousarray(a).view(np.float64)
+    with np.errstate(over="ignore", invalid="ignore"):
+        total = x.sum()
+    return bool(np.isfinite(total)) or bool(np.isfinite(x).all())
+
+
 def calculate_timeseries_cpp(grid, sbus_matrix, tolerance: float = 1e-8, max_iterations: int = 30,
                              n_threads: int = 0, init: str = "dc", precision: str = "double", solver=None,
                              dc_stamps=None, p_shift=None):
@@ -137,7 +147,7 @@ def calculate_timeseries_cpp(grid, sbus_matrix, tolerance: float = 1e-8, max_ite
         raise ValueError("Network has no buses")
     if T == 0:
         raise ValueError("Time series has zero time steps")
-    if np.any(np.isnan(S)) or np.any(np.isinf(S)):
+    if not _all_finite(S):
         raise ValueError("Sbus matrix contains NaN or inf values")
     if solver is None:
         solver = PolarNewtonSolverCUDA(grid.Yp, grid.Yj, grid.Yx, grid.pv, grid.pq)
@@ -146,13 +156,13 @@ def calculate_timeseries_cpp(grid, sbus_matrix, tolerance: float = 1e-8, max_ite
         is_slack[np.asarray(grid.ref, dtype=np.int64)] = 1
         solver._s.set_branches(grid.f, grid.t, grid.stamp_pos, grid.stamp, is_slack)
     v_init = _start_voltage(grid, init, solver._s, dc_stamps, p_shift)
-    if np.any(np.isnan(v_init)) or np.any(np.isinf(v_init)):
+    if not _all_finite(v_init):
         raise ValueError("DC initial voltage contains NaN or inf values")
     if v_init.shape[0] != n_bus:
         raise ValueError(f"V0 shape mismatch: expected ({n_bus},), got {v_init.shape}")
     solver.precision = precision
     result = solver.solve_batch(S, v_init, max_iter=max_iterations, tol=tolerance)
-    if np.any(np.isnan(result["V"])) or np.any(np.isinf(result["V"])):
+    if not _all_finite(result["V"]):
         raise ValueError("batch solver returned NaN or inf voltages")
     if not bool(np.all(result["converged"])):
         n_bad = int((~np.asarray(result["converged"], bool)).sum())

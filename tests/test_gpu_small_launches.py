@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from oracle import cpu
+from p3s_gb300.group import GpuGroup, GroupJob
 from p3s_gb300.solver import GpuSolver
 from p3s_gb300.synthetic import make_grid, scenario_injections
 
@@ -53,3 +54,39 @@ def test_shared_start_where_it_pays_changes_no_result(cases):
             assert np.array_equal(r[how]["V"], r[True]["V"])
             assert np.array_equal(r[how]["iterations"], r[True]["iterations"])
         assert r[True]["converged"].all()
+
+
+@pytest.mark.parametrize("cases", [3084, 3085, 52428, 52429])
+def test_results_by_the_staging_block_and_directly(cases):
+    """5 buses: voltages, iterations and flags of 3,084 cases fit the page-locked block, of 3,085 only the
+    iterations and flags, of 52,429 nothing: the same bits from each, for a solver and a group."""
+    g = make_grid(5, seed=5, max_drop_pu=0.05)
+    S3 = scenario_injections(g, 3, seed=2)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    p = GpuSolver.params()
+    want = s.solve_batch(S3, g.V0, p)
+    S = np.ascontiguousarray(S3[:, np.arange(cases) % 3])
+    grp = GpuGroup()
+    few, many = grp.solve([GroupJob(s, S3, g.V0), GroupJob(s, S, g.V0)], p)
+    for got in (s.solve_batch(S, g.V0, p), many):
+        assert np.array_equal(got["V"], want["V"][:, np.arange(cases) % 3])
+        assert np.array_equal(got["iterations"], want["iterations"][np.arange(cases) % 3])
+        assert got["converged"].all()
+    assert np.array_equal(few["V"], want["V"]) and few["converged"].all()
+
+
+def test_dc_starts_share_work_arrays():
+    """Few, many (work arrays freed after the call) and few cases again, with and without DC stamps."""
+    g = make_grid(257, seed=257, max_drop_pu=0.05)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    is_slack = np.zeros(g.n, np.uint8)
+    is_slack[np.asarray(g.ref)] = 1
+    s.set_branches(g.f, g.t, g.stamp_pos, g.stamp, is_slack)
+    P3 = np.ascontiguousarray(scenario_injections(g, 3, seed=4).real)
+    for stamps in (None, g.stamp):
+        want = [s.dc_start(np.ascontiguousarray(P3[:, k]), g.V0, dc_stamps=stamps)[0] for k in range(3)]
+        for cases in (3, 17000, 3):
+            V, used = s.dc_start(np.ascontiguousarray(P3[:, np.arange(cases) % 3]), g.V0, dc_stamps=stamps)
+            assert used.all()
+            for k in range(3):
+                assert np.array_equal(V[:, k::3], np.repeat(want[k][:, None], len(range(k, cases, 3)), axis=1))
