@@ -2293,7 +2293,7 @@ int gbpf_stream_submit(gbpf_stream* st, const gbpf_job* J) {
                                 reinterpret_cast<int*>(dscr), reinterpret_cast<unsigned long long*>(dbest),
                                 reinterpret_cast<int*>(dlab), reinterpret_cast<uint8_t*>(dsv),
                                 reinterpret_cast<int*>(dref), reinterpret_cast<int*>(dni), st->derr() + 6, igrid,
-                                st->sub));
+                                st->sub, /*beside_resident=*/true));
         if (J->served) CK(cudaMemcpyAsync(J->served, dsv, n * T, cudaMemcpyDeviceToHost, st->sub));
         b.ymode = 3;
         b.out_ptr = reinterpret_cast<const int*>(dop);

@@ -243,7 +243,7 @@ cudaError_t launch_ybus_gather(int nnz, int m4, const int* ptr, const int* src, 
 cudaError_t launch_islands(int n, int m, const int* f, const int* t, const uint8_t* live, int L, const int* out_ptr,
                            const int* out_idx, const uint8_t* is_slack, const double* prio, int reslack, int* scratch,
                            unsigned long long* best, int* labels, uint8_t* served, int* ref_bus, int* n_islands,
-                           int* err, int grid, cudaStream_t stream);
+                           int* err, int grid, cudaStream_t stream, bool beside_resident = false);
 // Load a kernel's code into the context now (cudaFuncGetAttributes). With lazy module loading
 // a kernel is otherwise loaded at its first launch, and loading waits for the kernels running on
 // the device -- for a stream launch, until it ends; the stream launch preloads every kernel that

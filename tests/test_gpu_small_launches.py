@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 
 from oracle import cpu
+from oracle import islands as oislands
+from p3s_gb300 import contingency
 from p3s_gb300.group import GpuGroup, GroupJob
 from p3s_gb300.solver import GpuSolver
 from p3s_gb300.synthetic import make_grid, scenario_injections
@@ -90,3 +92,25 @@ def test_dc_starts_share_work_arrays():
             assert used.all()
             for k in range(3):
                 assert np.array_equal(V[:, k::3], np.repeat(want[k][:, None], len(range(k, cases, 3)), axis=1))
+
+
+@pytest.mark.parametrize("n,cases", [(1, 1), (4, 7), (28, 8), (29, 9), (36, 17), (37, 3), (1000, 33),
+                                     (1256, 9), (1257, 9), (2536, 5), (2537, 5), (4096, 5), (4097, 5)])
+def test_islands_at_the_edges_of_both_kernels(n, cases):
+    """Labels in shared memory with four, two and one case a CTA up to 1,256, 2,536 and 4,096 buses, in
+    global memory beyond: random graphs with many components, self-loops, parallel and dead branches,
+    equal priorities."""
+    rng = np.random.default_rng(n + cases)
+    m = int(1.1 * n)
+    f, t = rng.integers(0, n, m).astype(np.int32), rng.integers(0, n, m).astype(np.int32)
+    t[: m // 2] = np.minimum(f[: m // 2] + 1, n - 1)  # long chains: the deepest trees
+    live = rng.random(m) < 0.9
+    groups = [rng.choice(m, size=min(m, int(rng.integers(0, 4))), replace=False) for _ in range(cases)]
+    prio = rng.integers(-1, 3, n).astype(float)
+    ref = np.unique(rng.integers(0, n, max(1, n // 50)))
+    batch = contingency.ContingencyBatch(None, None, None, n, groups, None, None, ref, f, t, live, None)
+    for reslack in (True, False):
+        got = contingency.islands(batch, reslack, prio)
+        want = oislands.islands(n, f, t, live, groups, ref, reslack, prio)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
