@@ -661,6 +661,7 @@ int enqueue_launch(gbpf_solver* s, LaunchRes& R, gbpf::Batch& b, long long units
     L.cta_bytes = job.off.total;
     L.timed = b.timers;
     L.mixed = b.mixed;
+    L.stamp_slots = b.ymode == 1 || b.ymode == 3 ? G : 0;
     CK(cudaEventRecord(R.e0, R.stream));
     if (b.v0_shared)
         CK(gbpf::launch_v0_table(b.V0, s->n, b.check_v0, R.btab->as<double4_32a>(), b.err, R.stream));
@@ -1000,6 +1001,8 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     L.scratch = g->scr.as<char>();
     L.cta_bytes = cta_bytes;
     L.mixed = mixed;
+    for (const gbpf::Job& o : hj)
+        if (o.B.ymode == 1 || o.B.ymode == 3) L.stamp_slots = std::max(L.stamp_slots, o.G);
     CK(cudaEventRecord(g->e0, g->stream));
     for (int q = 0; q < nj; ++q) {
         const gbpf::Batch& b = hj[q].B;
@@ -2165,6 +2168,7 @@ int gbpf_stream_start(gbpf_stream* st, int nsolvers, gbpf_solver* const* solvers
     L.njobs = st->capacity;
     L.scratch = st->scr.as<char>();
     L.cta_bytes = cta;
+    L.stamp_slots = gbpf::MAX_SLOTS;  // jobs to come may have stamps
     L.ring.published = st->dctl();
     L.ring.stop = st->dctl() + 1;
     L.ring.status = st->dctl() + 2;

@@ -190,6 +190,7 @@ struct Launch {
     unsigned long long cta_bytes;
     int mixed;               // its jobs' precision (a stream launch's jobs each have their own)
     int timed;               // the instantiation that counts SM cycles per phase (stats[8 .. 13])
+    int stamp_slots;         // largest slot count of its jobs with outage stamps (0: none has any)
     Ring ring;
 };
 

@@ -1051,7 +1051,13 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
     __shared__ DevPlan s_plan1;  // the same topology with the one-slot schedule (solo passes)
     __shared__ Batch s_batch;
     __shared__ int s_solo;
-    __shared__ double4_32a s_dinv64[NTB];  // double passes: each worker's inverse diagonal (off the registers)
+    // double passes: each worker's inverse diagonal, off the registers. A mixed launch makes few of
+    // them and leaves it to the registers and their spills: without these 32 bytes a thread and with
+    // the stamps below only where there are any, its CTAs take 6 KB of shared memory and not 27 to 59,
+    // the rest is L1: 19,999 buses x 16 cases 6.82 -> 6.59 ms, 777 x 96 1.00 -> 0.96, 2,000 x 8,760
+    // in lanes 29.1 -> 28.4 (a double launch gains nothing by it)
+    __shared__ double4_32a s_dinv64[PREC == 1 ? 1 : NTB];
+    double4_32a* const dinv64 = PREC == 1 ? nullptr : s_dinv64;
     __shared__ int s_job;
     __shared__ ScratchOffsets s_off;
     __shared__ int s_G, s_lg, s_fin;
@@ -1145,8 +1151,9 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
     // their threads to those slots only (see `lanes_of`)
     __shared__ int s_act[MAX_SLOTS], s_nact;
     __shared__ int s_share;  // the launch's shared start is usable (its factorization passed)
-    __shared__ int s_stk[MAX_SLOTS][MAX_STAMPS];
-    __shared__ double2 s_stv[MAX_SLOTS][MAX_STAMPS];
+    // outage stamps of every slot (entry values, then rows), only in launches that have any
+    extern __shared__ double2 s_stv[];
+    int* const s_stk = reinterpret_cast<int*>(s_stv + (MAX_STAMPS << lg));
     __shared__ unsigned long long s_ph[6];  // timed launches: SM cycles per phase of this CTA and job
     __shared__ long long s_clk;
 
@@ -1252,14 +1259,14 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                                 continue;
                             }
                             const int4 pos = P.br_pos[b];
-                            s_stk[s][nst] = pos.x;
-                            s_stv[s][nst++] = P.br_val[4 * b];
-                            s_stk[s][nst] = pos.y;
-                            s_stv[s][nst++] = P.br_val[4 * b + 1];
-                            s_stk[s][nst] = pos.z;
-                            s_stv[s][nst++] = P.br_val[4 * b + 2];
-                            s_stk[s][nst] = pos.w;
-                            s_stv[s][nst++] = P.br_val[4 * b + 3];
+                            s_stk[s * MAX_STAMPS + nst] = pos.x;
+                            s_stv[s * MAX_STAMPS + nst++] = P.br_val[4 * b];
+                            s_stk[s * MAX_STAMPS + nst] = pos.y;
+                            s_stv[s * MAX_STAMPS + nst++] = P.br_val[4 * b + 1];
+                            s_stk[s * MAX_STAMPS + nst] = pos.z;
+                            s_stv[s * MAX_STAMPS + nst++] = P.br_val[4 * b + 2];
+                            s_stk[s * MAX_STAMPS + nst] = pos.w;
+                            s_stv[s * MAX_STAMPS + nst++] = P.br_val[4 * b + 3];
                         }
                     } else if (Bt.ymode == 1) {
                         const int e0 = Bt.st_ptr[c], e1 = Bt.st_ptr[c + 1];
@@ -1272,8 +1279,8 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                             nst = MAX_STAMPS;
                         }
                         for (int e = 0; e < nst; ++e) {
-                            s_stk[s][e] = Bt.st_k[e0 + e];
-                            s_stv[s][e] = Bt.st_v[e0 + e];
+                            s_stk[s * MAX_STAMPS + e] = Bt.st_k[e0 + e];
+                            s_stv[s * MAX_STAMPS + e] = Bt.st_v[e0 + e];
                         }
                     }
                     s_nst[s] = nst;
@@ -1436,7 +1443,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                 const int s = idx & (G - 1);
                 if (!(s_on32[s] && !s_nofac[s] && s_nojac[s])) continue;
                 const int4 rec = __ldg(&P.rows[idx >> lg]);
-                EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, s_case[s], s_nst[s], s_stk[s], s_stv[s]};
+                EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, s_case[s], s_nst[s], s_stk + s * MAX_STAMPS, s_stv + s * MAX_STAMPS};
                 eval_row<2>(ec, rec, s, spin[((size_t)rec.x << lg) + s] != 0, make_double2(0.0, 0.0),
                             s_fb[s] ? fac32 : fac32b, R, false);
             }
@@ -1488,7 +1495,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
                 const int s = idx & (G - 1);
                 if (!s_reeval[s]) continue;
                 const int4 rec = __ldg(&P.rows[idx >> lg]);
-                EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, s_case[s], s_nst[s], s_stk[s], s_stv[s]};
+                EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, s_case[s], s_nst[s], s_stk + s * MAX_STAMPS, s_stv + s * MAX_STAMPS};
                 eval_row<1>(ec, rec, s, spin[((size_t)rec.x << lg) + s] != 0, make_double2(0.0, 0.0), fac64, R, false);
             }
             __syncthreads();
@@ -1503,10 +1510,10 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             double4_32a* const fd = s_first[sl] ? (double4_32a*)Bt.fac0 : fac64;
             if constexpr (PREC == 0)
                 lu_pass<double, TIMED>(solo >= 0 ? s_plan1 : P, fd, R, y64, s_on64, lg, s_pmin, s_pmax, nofac, !all_first,
-                                       s_dinv64, solo, GBPF_PH, &s_clk);
+                                       dinv64, solo, GBPF_PH, &s_clk);
             else
                 lu_pass<double, TIMED, false>(solo >= 0 ? s_plan1 : P, fd, R, y64, s_on64, lg, s_pmin, s_pmax, nofac,
-                                              !all_first, s_dinv64, solo, GBPF_PH, &s_clk);
+                                              !all_first, dinv64, solo, GBPF_PH, &s_clk);
             if (tid < G && s_on64[tid]) {
                 const int s = tid;
                 if (s_nofac[s]) {
@@ -1677,7 +1684,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
             const int c = s_case[s];
             const double2 Ssp = ld_in<RING>(Bt.s_shared ? Bt.S + bus : Bt.S + (size_t)bus * Bt.sS + c);
             const bool pinned = spin[((size_t)bus << lg) + s] != 0;
-            EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, c, s_nst[s], s_stk[s], s_stv[s]};
+            EvalCtx ec{&P, Et, Ei, iv32, lg, Bt.ymode == 3 ? 1 : Bt.ymode, Bt.Yd, Bt.sYd, c, s_nst[s], s_stk + s * MAX_STAMPS, s_stv + s * MAX_STAMPS};
             unsigned long long worst = 0ULL;
             if (st == SL_BACKTRACK || (mixed && s_jprec[s] && s_nojac[s]))  // the mismatch only (line search, lazy Jacobian)
                 worst = eval_row<0>(ec, rec, s, pinned, Ssp, fac64, R, true);
@@ -2131,34 +2138,34 @@ __global__ void eval_debug_kernel(const DevPlan P, const double2* V, const doubl
     }
 }
 
+template <int NTB, bool TIMED, bool RING, int PREC>
+static cudaError_t start_one(const Launch& L, int grid, cudaStream_t stream) {
+    auto* k = newton_kernel<NTB, TIMED, RING, PREC>;
+    const int slot = MAX_STAMPS * (int)(sizeof(double2) + sizeof(int));
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SLOTS * slot);
+    if (e) return e;
+    k<<<grid, NTB, L.stamp_slots * slot, stream>>>(L);
+    return cudaGetLastError();
+}
+
 template <int NTB>
-static void start_newton(const Launch& L, int grid, cudaStream_t stream) {
+static cudaError_t start_newton(const Launch& L, int grid, cudaStream_t stream) {
     if (L.mixed)
-        L.timed ? newton_kernel<NTB, true, false, 1><<<grid, NTB, 0, stream>>>(L)
-                : newton_kernel<NTB, false, false, 1><<<grid, NTB, 0, stream>>>(L);
-    else
-        L.timed ? newton_kernel<NTB, true, false, 0><<<grid, NTB, 0, stream>>>(L)
-                : newton_kernel<NTB, false, false, 0><<<grid, NTB, 0, stream>>>(L);
+        return L.timed ? start_one<NTB, true, false, 1>(L, grid, stream) : start_one<NTB, false, false, 1>(L, grid, stream);
+    return L.timed ? start_one<NTB, true, false, 0>(L, grid, stream) : start_one<NTB, false, false, 0>(L, grid, stream);
 }
 
 cudaError_t launch_newton(const Launch& L, int grid, int threads, cudaStream_t stream) {
     if (L.ring.published) {  // a stream launch: untimed
         if (L.timed) return cudaErrorInvalidValue;
-        if (threads == 1024)
-            newton_kernel<1024, false, true, 2><<<grid, 1024, 0, stream>>>(L);
-        else if (threads == 512)
-            newton_kernel<512, false, true, 2><<<grid, 512, 0, stream>>>(L);
-        else
-            return cudaErrorInvalidValue;
-    } else if (threads == 1024)
-        start_newton<1024>(L, grid, stream);
-    else if (threads == 512)
-        start_newton<512>(L, grid, stream);
-    else if (threads == 256)
-        start_newton<256>(L, grid, stream);
-    else
+        if (threads == 1024) return start_one<1024, false, true, 2>(L, grid, stream);
+        if (threads == 512) return start_one<512, false, true, 2>(L, grid, stream);
         return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    }
+    if (threads == 1024) return start_newton<1024>(L, grid, stream);
+    if (threads == 512) return start_newton<512>(L, grid, stream);
+    if (threads == 256) return start_newton<256>(L, grid, stream);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_eval_debug(const DevPlan& P, const double2* V, const double2* Sbus, const uint8_t* pin,

@@ -114,3 +114,29 @@ def test_islands_at_the_edges_of_both_kernels(n, cases):
         want = oislands.islands(n, f, t, live, groups, ref, reslack, prio)
         for a, b in zip(got, want):
             assert np.array_equal(a, b)
+
+
+def test_stamps_beside_plain_jobs_of_other_slot_counts():
+    """A group launch's outage stamps lie behind the slots of each job: an outage job of few slots beside a
+    plain one of many, and the other way round, give the bits of each job alone."""
+    g = make_grid(65, seed=65, max_drop_pu=0.05)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    is_slack = np.zeros(g.n, np.uint8)
+    is_slack[np.asarray(g.ref)] = 1
+    s.set_branches(g.f, g.t, g.stamp_pos, g.stamp, is_slack, np.maximum(g.p_gen, 0.0))
+    S = scenario_injections(g, 40, seed=6)
+    groups = [[], *[[b] for b in range(39)]]
+    out = contingency.outage_lists(groups)
+    grp = GpuGroup()
+    for precision in ("double", "mixed"):
+        p = GpuSolver.params(precision=precision)
+        for few, many in ((1, 32), (32, 1), (4, 4)):
+            jobs = [GroupJob(s, S, g.V0, cases_per_cta=many),
+                    GroupJob(s, np.asarray(g.Sbus), g.V0, n_cases=40, outages=out, reslack=True, cases_per_cta=few)]
+            both = grp.solve(jobs, p)
+            for r, job in zip(both, jobs):
+                alone = grp.solve([job], p)[0]
+                assert np.array_equal(r["V"], alone["V"], equal_nan=True)
+                assert np.array_equal(r["iterations"], alone["iterations"])
+                assert np.array_equal(r["converged"], alone["converged"])
+        assert not np.array_equal(both[1]["V"][:, 1], both[1]["V"][:, 0])
