@@ -521,6 +521,23 @@ struct Pivots<double> {
     __device__ __forceinline__ unsigned long long hi_bits() const { return hi; }
 };
 
+// A record of the schedule, read once a pass by one warp. With one slot a CTA (`first`) the records
+// are as many bytes as the factors, so they are marked to leave L1 before the factor blocks do; from
+// two slots on the factors outgrow L1 anyway, and there the mark costs (2,000 buses x 8,760 cases in
+// lanes: 28.3 ms, 29.8 with it). The branch alone is worth 1-5 % at every slot count, by where the
+// compiler then places the fetch. Before and after: 777 buses x 96 cases 1.00 and
+// 0.90 ms, one 2,000-bus case 1.71 and 1.63, 19,999 x 16 6.49 and 6.35, 2,000 x 8,760 9.4 and 9.2, in
+// lanes 28.2 and 27.2 ms. Equal or slower: the mark on the pairs too, on the evaluation's rows, from
+// 4 or 8 slots down, and volatile loads.
+__device__ __forceinline__ int4 ld_record(const int4* p, bool first) {
+    if (!first) return __ldg(p);
+    int4 v;
+    asm("ld.global.nc.L1::evict_first.v4.s32 {%0, %1, %2, %3}, [%4];"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+        : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+
 // What a pass's levels have in common: the slot of this lane, whether it takes part and whether
 // it factors, and how a warp's lanes are shared out (solo: the CTA's one slot left, all lanes).
 struct LuLane {
@@ -528,6 +545,7 @@ struct LuLane {
     int ll;            // slots side by side in a warp (log2; solo 0)
     int s;
     bool act, factor, factor_any;
+    bool first;        // records leave L1 before factor blocks
 };
 
 // Levels h0 .. h1 - 1 of the factorization and forward substitution, one lane a task.
@@ -556,8 +574,12 @@ __device__ __forceinline__ void lane_forward(const DevPlan& P, const LuLane& L, 
     int4 next = make_int4(-1, 0, 0, 0), nhead = next;
     auto fetch = [&](const int4* task) {
         const int4* rec = task + 2 * (((size_t)t << lgw) + wi);
-        next = __ldg(rec);
-        if constexpr (HEAD) nhead = __ldg(rec + 1);
+        if constexpr (HEAD) {
+            next = ld_record(rec, L.first);
+            nhead = ld_record(rec + 1, L.first);
+        } else {
+            next = __ldg(rec);
+        }
     };
     if (act) {
         const int* ptr = (factor_any ? P.ptrA : P.ptrF) + warp * (P.nlev + 1) + h0;
@@ -714,8 +736,12 @@ __device__ __forceinline__ void lane_backward(const DevPlan& P, const LuLane& L,
     int4 next = make_int4(-1, 0, 0, 0), nhead = next;
     auto fetch = [&](const int4* task) {
         const int4* rec = task + 2 * (((size_t)t << lgw) + wi);
-        next = __ldg(rec);
-        if constexpr (HEAD) nhead = __ldg(rec + 1);
+        if constexpr (HEAD) {
+            next = ld_record(rec, L.first);
+            nhead = ld_record(rec + 1, L.first);
+        } else {
+            next = __ldg(rec);
+        }
     };
     if (act) {
         const int* ptr = P.ptrC + warp * (P.nblev + 1) + h0;
@@ -1006,6 +1032,7 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
     L.act = on[L.s] != 0;
     L.factor = !(chord && chord[L.s]);
     L.factor_any = factor_any;
+    L.first = sizeof(real) == 4 && lg == 0;
     Pivots<real> pv;
     if constexpr (sizeof(real) == 8 && QUADS) {
         const int hq = factor_any ? P.quad_from : P.nlev;
