@@ -353,9 +353,20 @@ __device__ unsigned long long eval_row(const EvalCtx& c, int4 rec, int s, bool p
 }
 
 // Reciprocal of a positive double: float seed refined by two Newton-Raphson steps
-// r <- r (2 - x r) (quadratic convergence: ~2^-24 -> 2^-48 -> below double rounding).
+// r <- r (2 - x r) (quadratic convergence: ~2^-24 -> 2^-48 -> below double rounding). Between
+// 2^-31 and 2^31, where magnitudes lie, the seed's two conversions are made on the integer pipes
+// (round to nearest even, the same bits): a double update is bound by its FP64 instructions, ~30 a
+// bus of which these were two.
 __device__ __forceinline__ double recip_nr(double x) {
-    double r = (double)__frcp_rn((float)x);
+    double r;
+    const unsigned hi = (unsigned)__double2hiint(x);
+    if (hi - 0x3e000000u < 0x03e00000u) {
+        const unsigned long long u = dbits(x) + 0x0fffffffULL + ((dbits(x) >> 29) & 1ULL);
+        const unsigned b = __float_as_uint(__frcp_rn(__uint_as_float((unsigned)(u >> 29) - (896u << 23))));
+        r = __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
+    } else {
+        r = (double)__frcp_rn((float)x);
+    }
     r = r * fma(-x, r, 2.0);
     r = r * fma(-x, r, 2.0);
     return r;

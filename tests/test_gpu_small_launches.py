@@ -3,12 +3,14 @@ grids around the sizes where levels change over, 1 to 8 slots a CTA, both precis
 CTA shape forms the same numbers, so a case's result must be bit-identical whatever its launch,
 and within the double path's 1e-11 of the oracle."""
 
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
 from oracle import cpu
 from oracle import islands as oislands
-from p3s_gb300 import contingency
+from p3s_gb300 import _lib, contingency
 from p3s_gb300.group import GpuGroup, GroupJob
 from p3s_gb300.solver import GpuSolver
 from p3s_gb300.synthetic import make_grid, scenario_injections
@@ -140,3 +142,22 @@ def test_stamps_beside_plain_jobs_of_other_slot_counts():
                 assert np.array_equal(r["iterations"], alone["iterations"])
                 assert np.array_equal(r["converged"], alone["converged"])
         assert not np.array_equal(both[1]["V"][:, 1], both[1]["V"][:, 0])
+
+
+@pytest.mark.parametrize("exponent", [-126, -32, -31, -1, 0, 1, 30, 31, 125])
+def test_reciprocal_seed_is_rounded_to_nearest(exponent):
+    """Inside and outside the range whose seed is converted on the integer pipes (2^-31 to 2^31): the bits
+    of a float reciprocal of the nearest float, refined by two fused Newton steps; ties, carries into the
+    exponent and neighbours of powers of two."""
+    rng = np.random.default_rng(exponent + 200)
+    man = np.concatenate([rng.integers(0, 1 << 52, 200), rng.integers(0, 1 << 23, 50) << 29,
+                          (rng.integers(0, 1 << 23, 50) << 29) + (1 << 28), [0, 1, (1 << 52) - 1, (1 << 28) - 1, 1 << 28]])
+    x = np.ldexp(1.0 + man.astype(np.float64) * 2.0 ** -52, exponent)
+    outs = [np.empty(len(x)) for _ in range(5)]
+    rc = _lib.load().gbpf_selftest_math(_lib.d(x), len(x), *[_lib.d(o) for o in outs], None, None)
+    assert rc == 0, _lib.last_error()
+    seed = (np.float32(1.0) / x.astype(np.float32)).astype(np.float64)
+    for a, r, got in zip(x, seed, outs[0]):
+        for _ in range(2):
+            r = float(r) * float(2 - Fraction(float(a)) * Fraction(float(r)))
+        assert got == r
