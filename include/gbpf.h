@@ -133,8 +133,8 @@ int gbpf_get_mismatch(gbpf_solver* s, double* out, long long n);
 int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta);
 int gbpf_set_shape(gbpf_solver* s, long long units, int threads_per_cta, int cases_per_cta);
 /* Builds, ahead of use, the schedules of every CTA shape a launch of this topology may take
- * with up to max_cases_per_cta slots (512 threads: 1, 2, 4, ... slots; 1,024: up to 4), so that
- * no later launch builds one on its critical path (a serving loop's warm-up). No reference
+ * with up to max_cases_per_cta slots (256 threads: up to 8 slots; 512 and 1,024: up to 32), so
+ * that no later launch builds one on its critical path (a serving loop's warm-up). No reference
  * counterpart. */
 int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta);
 /* Factorization schedule knob (no reference counterpart; the reference deals each level's

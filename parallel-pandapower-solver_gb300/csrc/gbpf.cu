@@ -324,23 +324,35 @@ int size_class(long long units) {
     return c;
 }
 
-// CTA shape for a batch of `units` cases of one grid (measured on GB300, 118 to 3,500 buses, 700
-// to 8,760 cases). Case slots per SM: the batch's share of an SM rounded up to a power of two, at
-// most 64 (32 above 4,096 variable buses, 16 above 16,384: the per-slot working set grows with the
-// grid). Up to 4 slots per SM run as one 1,024-thread CTA (many workers per case), more as two
-// 512-thread CTAs whose phases overlap -- except:
+// CTA shape for a batch of `units` cases of one grid (measured on GB300, 14 to 6,000 buses, 1 to
+// 8,760 cases). Case slots per SM: the batch's share of an SM rounded up to a power of two, at most
+// 64 (32 above 4,096 variable buses, 16 above 16,384: the per-slot working set grows with the grid).
+// One or two slots per SM run as one 1,024-thread CTA (many workers per case) from 600 variable
+// buses on, more as two 512-thread CTAs whose phases overlap -- except:
+// * one or two slots on smaller grids, whose narrow levels wait for the CTA's barrier and not for
+//   workers: 256 threads (mixed up to 250 buses, double up to 64) or 512 (double with one slot, both
+//   with two). One case: 118 buses mixed 0.241 -> 0.216 ms, double 0.337 -> 0.315, 14 buses 0.082 ->
+//   0.074; 300 cases of 118 buses 0.289 -> 0.270, of 490 double 0.870 -> 0.860. At 300 buses mixed
+//   256 threads take 0.280 where 1,024 take 0.260.
+// * a share of three cases: three of four 256-thread CTAs with a slot each, in lanes above all (2,000
+//   buses, 400 lanes of 12: mixed 20.9 -> 16.1 ms, double 30.7 -> 25.8; 456 cases at once 1.45 -> 1.41
+//   and 2.41 -> 2.13). Above 4,096 variable buses a mixed case misses the workers (456 cases of 6,000
+//   buses 4.07 ms): there three or four slots run as one 1,024-thread CTA (3.78).
+// * mixed, 8 to 32 slots per SM of which at most three quarters are needed: three of four
+//   256-thread CTAs (490 buses, 744 cases 0.85 -> 0.83 ms, 3,001 cases 1.67 -> 1.60), but for 32
+//   slots on larger grids, for which the next rule holds (2,000 buses, 1,600 cases 3.13 -> 3.01, but
+//   3,001 cases 4.72 -> 4.91).
 // * mixed, 8 to 32 slots per SM on larger grids (from 24,000 buses x slots on): one 1,024-thread
 //   CTA. Twice the workers on one slot set shorten the waits that bound a pass there (2,000 buses,
 //   3,001 cases: 5.25 -> 4.93 ms; 3,500 buses, 2,432 cases 5.1 -> 4.6), below it they are equal.
-// * mixed, 8 to 32 slots per SM of which at most three quarters are needed: three of four
-//   256-thread CTAs (490 buses, 744 cases 0.85 -> 0.83 ms, 3,001 cases 1.67 -> 1.60).
 // * double: the FP64 pipes are the bound, and they take a warp's time for however few of its
 //   lanes work, so a rounded-up share is paid for in full. The shape with the fewest slots on
 //   the fullest SM: CTAs not all resident at once are refilled and share the cases evenly, at
 //   the price of about one more CTA's slots at the end (on grids below 400 buses of far more);
 //   32-slot CTAs (a worker a warp, no divergence) do a slot's work in 0.84 of the time, 4- and
 //   2-slot ones in 1.12 and 1.25, and eight slots in all leave an SM waiting; one CTA of fewer
-//   than 1,024 threads alone on its SM takes 1.05. 2,000 buses: 744 cases 3.58 -> 3.14 ms, 3,001
+//   than 1,024 threads alone on its SM takes 1.15 (1,216 cases of 2,000 buses on 512 threads: 8 slots
+//   3.81 ms, two CTAs of 4 slots 3.57; 490 buses 1.39 and 1.38). 2,000 buses: 744 cases 3.58 -> 3.14 ms, 3,001
 //   cases 10.7 -> 8.6, 6,000 cases 17.8 -> 14.0; 490 buses, 3,001 cases 3.1 -> 2.6.
 // * outage cases take unlike numbers of passes, so slots that refill pay more: double counts
 //   half a CTA's slots on top, and a CTA holds at most 8,192 buses x slots (2,000-bus N-1 sweep:
@@ -350,9 +362,15 @@ void batch_shape(int nsm, int nv, long long units, bool mixed, bool outages, int
     const long long share = (units + nsm - 1) / nsm;
     int per_sm = 1;
     while (per_sm < share && per_sm < cap) per_sm *= 2;
-    if (per_sm <= 4) {
-        *NT = 1024;
+    if (share <= 2) {
+        const int few = mixed ? 250 : 64;
+        *NT = nv <= few ? 256 : nv <= 600 && !(mixed && share == 1) ? 512 : 1024;
         *G = per_sm;
+        return;
+    }
+    if (per_sm == 4) {
+        *NT = mixed && nv > 4096 ? 1024 : share == 3 ? 256 : 512;
+        *G = *NT == 1024 ? 4 : *NT == 512 ? 2 : 1;
         return;
     }
     auto fit_outages = [&]() {
@@ -362,7 +380,8 @@ void batch_shape(int nsm, int nv, long long units, bool mixed, bool outages, int
     };
     if (mixed) {
         const bool mid = per_sm <= 32;
-        *NT = mid && !outages && (long long)nv * per_sm >= 24000 ? 1024 : mid && 4 * share <= 3 * per_sm ? 256 : 512;
+        const bool three = mid && 4 * share <= 3 * per_sm, large = mid && !outages && (long long)nv * per_sm >= 24000;
+        *NT = large && !(three && per_sm < 32) ? 1024 : three ? 256 : 512;
         *G = std::min(gbpf::MAX_SLOTS, per_sm / (1024 / *NT));
         return fit_outages();
     }
@@ -378,7 +397,7 @@ void batch_shape(int nsm, int nv, long long units, bool mixed, bool outages, int
             double cost = refill ? (double)units / nsm + slots : per * slots + (outages ? 0.5 * slots : 0.0);
             cost *= slots == 32 ? 0.84 : slots == 4 ? (outages ? 1.05 : 1.12) : slots == 2 ? 1.25 : 1.0;
             if (refill && slots * on_sm == 8) cost *= 1.2;
-            if (per == 1 && on_sm > 1) cost *= 1.05;
+            if (per == 1 && on_sm > 1) cost *= 1.15;
             if (!*NT || cost < best) {
                 best = cost;
                 *NT = t;
@@ -1152,7 +1171,7 @@ int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta) {
     if (!s) return fail("null solver");
     const int cap = std::max(1, std::min(gbpf::MAX_SLOTS, max_cases_per_cta));
     for (int NT : {1024, 512, 256})
-        for (int G = NT == 256 ? 2 : 1; G <= (NT == 256 ? std::min(cap, 8) : cap); G *= 2) {  // (batch_shape's)
+        for (int G = 1; G <= (NT == 256 ? std::min(cap, 8) : cap); G *= 2) {  // (batch_shape's)
             Shape* sh = nullptr;
             if (int rc = get_shape(s, NT, G, &sh)) return rc;
         }

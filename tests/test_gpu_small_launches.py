@@ -161,3 +161,22 @@ def test_reciprocal_seed_is_rounded_to_nearest(exponent):
         for _ in range(2):
             r = float(r) * float(2 - Fraction(float(a)) * Fraction(float(r)))
         assert got == r
+
+
+@pytest.mark.parametrize("n", [14, 65, 257, 617])
+@pytest.mark.parametrize("cases", [1, 153, 305, 457])
+def test_shapes_of_small_shares_agree_bit_for_bit(n, cases):
+    """One to four cases an SM on grids below and above the lines between 256, 512 and 1,024 threads: the
+    chosen shape's results are those of one 1,024-thread CTA with four slots."""
+    g = make_grid(n, seed=n, max_drop_pu=0.05)
+    S = scenario_injections(g, cases, seed=n)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    for precision in ("double", "mixed"):
+        p = GpuSolver.params(precision=precision)
+        auto = s.solve_batch(S, g.V0, p)
+        s.set_shape(cases, 1024, 4)
+        r = s.solve_batch(S, g.V0, p)
+        s.set_shape(cases, 0, 0)
+        for key in ("V", "iterations", "converged"):
+            assert np.array_equal(auto[key], r[key])
+        assert auto["converged"].all()
