@@ -116,7 +116,7 @@ TUNE_SHAPES = ((512, 32), (512, 16), (1024, 32), (1024, 16))
 # ... of the uneven multi-grid launch: (threads per CTA, 0 = the rule; variable buses x case
 # slots a CTA takes per job, the group rule's 16,384 and its neighbours)
 MG_PACKING = ((0, 16384), (0, 8192), (0, 32768), (512, 4096), (1024, 16384))
-# ... and of the N-1 sweep's launch (3,001 cases; 0 = the group rule: 512 x 16)
+# ... and of the N-1 sweep's launch (3,001 cases; 0 = the rule of a group launch of one job)
 N1_SHAPES = ((0, 0), (512, 8), (512, 32), (1024, 8), (1024, 16), (256, 4), (256, 8))
 
 

@@ -21,8 +21,8 @@ enum SlotState : int {
 };
 
 constexpr int MAX_SLOTS = 32;    // cases per CTA (G) upper bound
-constexpr int QUAD_LG = 3;       // up to 2^3 slots a CTA: four lanes per factorization task (lu_quad)
-constexpr int MAX_STAMPS = 32;   // outage-stamp entries per case held in shared memory
+constexpr int QUAD_LG = 3;       // up to 2^3 slots a CTA: four lanes per factorization task (Quad)
+constexpr int MAX_STAMPS = 32;   // outage-stamp entries per case, held in dynamic shared memory
 
 // error codes written to Batch::err[0] (first error wins; err[1..2] = bus, case)
 enum DevError : int {

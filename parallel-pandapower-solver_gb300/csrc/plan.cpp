@@ -51,9 +51,9 @@ inline int rank_in(const std::vector<int>& Li, int lo, int hi, int x) {
     return (int)(std::lower_bound(Li.begin() + lo, Li.begin() + hi, x) - (Li.begin() + lo));
 }
 
-// Deal tasks (weights) of one level to W workers: longest first, each onto the currently
-// least-loaded worker (ties: lowest worker). Returns the worker of every task and the
-// largest worker load.
+// Deal bundles (weights) of one level to W warps: longest first, each onto the currently
+// least-loaded warp (ties: lowest warp). Returns the warp of every bundle and the largest
+// load of a warp.
 int deal(const std::vector<long long>& weight, int W, std::vector<int>& who) {
     const int n = (int)weight.size();
     std::vector<int> idx(n);

@@ -19,9 +19,11 @@
 //    Jacobian's diagonal block stays intact through the pass: a chain heavier than its
 //    level's share of a worker is cut into segments, each later segment led by a copy of
 //    the diagonal task that recomputes the inverse from it without storing anything. Tasks
-//    and chain segments are grouped by elimination-tree height (level) and dealt to the
-//    CTA's workers longest-first onto the least-loaded worker. The forward substitution
-//    rides along in the same levels.
+//    and chain segments are grouped by elimination-tree height (level), bundled with others of
+//    like length into steps of a warp, and the bundles dealt to the CTA's warps longest-first
+//    onto the least-loaded one (Schedule below). Pairs of a long task whose operands are final
+//    earlier are summed in an earlier level. The forward substitution rides along in the same
+//    levels.
 #pragma once
 
 #include <cstdint>

@@ -19,8 +19,8 @@ import numpy as np
 from .solver import GpuSolver
 from .synthetic import lanes
 
-CANDIDATES = ((1024, 1), (1024, 2), (1024, 4), (512, 2), (512, 4), (512, 8), (512, 16), (512, 32), (256, 4),
-              (256, 8), (256, 16))
+CANDIDATES = ((1024, 1), (1024, 2), (1024, 4), (512, 1), (512, 2), (512, 4), (512, 8), (512, 16), (512, 32),
+              (256, 1), (256, 2), (256, 4), (256, 8), (256, 16))
 
 
 CHAIN_CAPS = (1.0, 0.75, 0.5, 0.35, 0.25, 2.0, 0.0)
