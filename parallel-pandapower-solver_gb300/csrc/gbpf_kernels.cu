@@ -2182,21 +2182,10 @@ static cudaError_t start_one(const Launch& L, int grid, cudaStream_t stream) {
     const int slot = MAX_STAMPS * (int)(sizeof(double2) + sizeof(int));
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SLOTS * slot);
     if (e) return e;
-    // As much shared memory as the CTAs that the registers let reside (1,024 threads an SM) take,
-    // and a kilobyte each; left alone, the split has room for as many as 2,048 threads would be (102
-    // KB for double CTAs of 512 threads that take 46). One 118-bus double case 0.476 -> 0.444 ms, 490
-    // buses x 744 cases 3.53 -> 3.50, a 2,000-bus double N-1 sweep 23.55 -> 23.47, others equal. Where
-    // launches with and without stamps overlap the hint may be the other's: fewer CTAs reside then.
-    if (!RING) {
-        static const size_t fixed = [&]() -> size_t {
-            cudaFuncAttributes f;
-            return cudaFuncGetAttributes(&f, k) == cudaSuccess ? f.sharedSizeBytes : 0;
-        }();
-        const size_t need = (1024 / NTB) * (fixed + (size_t)L.stamp_slots * slot + 1024), all = 228 * 1024;
-        if (fixed && need <= all)
-            e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)((100 * need + all - 1) / all));
-        if (e) return e;
-    }
+    // (The split between shared memory and L1 is left to the driver, which keeps room for the CTAs
+    // of 2,048 threads an SM. An exact fit, cudaFuncAttributePreferredSharedMemoryCarveout, takes one
+    // 118-bus double case from 0.476 to 0.444 ms, but then no CTA of another launch gets in beside:
+    // four launch contexts in flight serve 280-400 requests/s instead of 560.)
     k<<<grid, NTB, L.stamp_slots * slot, stream>>>(L);
     return cudaGetLastError();
 }
