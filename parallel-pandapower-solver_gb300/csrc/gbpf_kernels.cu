@@ -1588,10 +1588,14 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         // grid (4 slots a CTA, 2.4 of them busy): evaluation 10.6 -> 9.2 ms mixed, 17.7 -> 13.0
         // ms double, with the rows by length below. From 16 slots on a warp keeps one or two
         // buses for its lanes, with few record loads, instead of straddling more (3,001 cases, 16
-        // slots, 10 busy: evaluation 1.93 ms mixed, 2.09 dealt; N-1 sweeps equal either way).
+        // slots, 10 busy: evaluation 1.93 ms mixed, 2.09 dealt; N-1 sweeps equal either way). One busy
+        // slot alone has all threads on any CTA: with its share of a full CTA, 16 of 512, an hour without
+        // a solution added 13.3 ms to a double series of 8,760 hours of 2,000 buses, and adds 2.4 (mixed
+        // 11.0 and 4.3).
+        auto dealt = [&]() { return s_nact <= 1 || (4 * s_nact <= 3 * G && G < 16); };
         auto deal = [&](int& slot, int& first, int& stride) {
-            const int na = s_nact;
-            if (4 * na <= 3 * G && G < 16) {
+            if (dealt()) {
+                const int na = s_nact;
                 const int per = NT / max(na, 1);
                 slot = tid < per * na ? s_act[tid % max(na, 1)] : -1;
                 first = tid / max(na, 1);
@@ -1713,7 +1717,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         {
             int s, first, stride;
             deal(s, first, stride);
-            const int4* const rows = G < 16 ? P.rows_by_len : P.rows;
+            const int4* const rows = G < 16 || dealt() ? P.rows_by_len : P.rows;
             const int st = s >= 0 ? s_st[s] : SL_EMPTY;
             if (st == SL_FRESH || st == SL_ACTIVE || st == SL_NEEDJ || st == SL_BACKTRACK)
         for (int k = first; k < P.nv; k += stride) {
