@@ -133,9 +133,10 @@ int gbpf_get_mismatch(gbpf_solver* s, double* out, long long n);
 int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta);
 int gbpf_set_shape(gbpf_solver* s, long long units, int threads_per_cta, int cases_per_cta);
 /* Builds, ahead of use, the schedules of every CTA shape a launch of this topology may take
- * with up to max_cases_per_cta slots (256 threads: up to 8 slots; 512 and 1,024: up to 32), so
- * that no later launch builds one on its critical path (a serving loop's warm-up). No reference
- * counterpart. */
+ * with up to max_cases_per_cta slots by the batch-size and group rules, in either precision, so
+ * that no later launch builds one on its critical path (a serving loop's warm-up); shapes that a
+ * caller sets (gbpf_set_shape, a fixed shape, threads of a group) are not among them. No
+ * reference counterpart. */
 int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta);
 /* Factorization schedule knob (no reference counterpart; the reference deals each level's
  * tasks to a fixed number of lists, lean_lu_plan.py:172-190): within a level, a pivot's chain
@@ -433,6 +434,12 @@ int gbpf_branch_flows_device(int nbr, int L, const int32_t* f, const int32_t* t,
                              const int32_t* out_idx, double* S_from, double* S_to, double* i_from, double* i_to,
                              double* i_max, double* loading, void* stream);
 
+/* Host-only view of the shape rules (runs without a GPU, for tests): the batch rule's CTA shape for
+ * `units` cases of a grid on n_sm SMs, and the (threads, slots) pairs that gbpf_prepare_shapes
+ * builds there (returns their number, shapes: 2 x max_shapes). No reference counterpart. */
+int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int outages, int* threads_per_cta,
+                        int* cases_per_cta);
+int gbpf_selftest_shapes(int n_sm, int n_var_bus, int max_cases_per_cta, int32_t* shapes, int max_shapes);
 /* Host-only check of the planner and the device schedule (runs without a GPU): plan for
  * `workers` workers, Jacobian at (Vm, Va) with injections S (n complex), the schedule
  * executed serially with a structural race check per level. dx (n x 2): Newton step per

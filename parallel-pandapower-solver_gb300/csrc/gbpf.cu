@@ -16,7 +16,9 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gbpf.h"
@@ -426,6 +428,31 @@ void choose_shape(const gbpf_solver* s, long long units, bool mixed, int* NT, in
     while (per_sm < share && per_sm < cap) per_sm *= 2;
     *NT = s->fixed_NT ? s->fixed_NT : 512;
     *G = s->fixed_G ? s->fixed_G : std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / *NT)));
+}
+
+// (threads, slots) of every CTA that launches of one grid take with up to `most` slots, but for
+// shapes that a caller sets: 512 threads with any number of slots and 1,024 with up to four by the
+// group rule, what batch_shape gives for any batch, and one slot of each of these sizes for a CTA's
+// last case. Batches are taken at every eighth of a case per SM; beyond 128 cases an SM the rule
+// gives one shape (its costs cross for the last time at 118).
+std::set<std::pair<int, int>> rule_shapes(int nsm, int nv, int most) {
+    std::set<std::pair<int, int>> out;
+    auto add = [&](int NT, int G) {
+        if (G > most) return;
+        out.insert({NT, G});
+        out.insert({NT, 1});
+    };
+    for (int G = 1; G <= gbpf::MAX_SLOTS; G *= 2) {
+        add(512, G);
+        if (G <= 4) add(1024, G);
+    }
+    for (int k = 1; k <= 8 * 128; ++k)
+        for (int how = 0; how < 4; ++how) {
+            int NT = 0, G = 0;
+            batch_shape(nsm, nv, ((long long)k * nsm + 7) / 8, how & 1, how & 2, &NT, &G);
+            add(NT, G);
+        }
+    return out;
 }
 
 // The schedule of one CTA shape: tasks dealt to NT / G workers, uploaded next to the
@@ -1169,13 +1196,30 @@ int gbpf_get_info(gbpf_solver* s, gbpf_info* o) {
 
 int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta) {
     if (!s) return fail("null solver");
-    const int cap = std::max(1, std::min(gbpf::MAX_SLOTS, max_cases_per_cta));
-    for (int NT : {1024, 512, 256})
-        for (int G = 1; G <= (NT == 256 ? std::min(cap, 8) : cap); G *= 2) {  // (batch_shape's)
-            Shape* sh = nullptr;
-            if (int rc = get_shape(s, NT, G, &sh)) return rc;
-        }
+    for (const auto& [NT, G] : rule_shapes(s->nsm, std::max(1, s->plan.nv), std::max(1, max_cases_per_cta))) {
+        Shape* sh = nullptr;
+        if (int rc = get_shape(s, NT, G, &sh)) return rc;
+    }
     return 0;
+}
+
+int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int outages, int* threads_per_cta,
+                        int* cases_per_cta) {
+    if (n_sm <= 0 || n_var_bus <= 0 || units <= 0 || !threads_per_cta || !cases_per_cta)
+        return fail("selftest_shape: invalid argument");
+    batch_shape(n_sm, n_var_bus, units, mixed != 0, outages != 0, threads_per_cta, cases_per_cta);
+    return 0;
+}
+
+int gbpf_selftest_shapes(int n_sm, int n_var_bus, int max_cases_per_cta, int32_t* shapes, int max_shapes) {
+    if (n_sm <= 0 || n_var_bus <= 0 || !shapes) return fail("selftest_shapes: invalid argument");
+    int k = 0;
+    for (const auto& [NT, G] : rule_shapes(n_sm, n_var_bus, std::max(1, max_cases_per_cta))) {
+        if (k == max_shapes) return fail("selftest_shapes: too many shapes");
+        shapes[2 * k] = NT;
+        shapes[2 * k++ + 1] = G;
+    }
+    return k;
 }
 
 int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta) {

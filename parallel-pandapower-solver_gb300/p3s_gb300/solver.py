@@ -177,8 +177,8 @@ class GpuSolver:
         return nt.value, g.value
 
     def prepare_shapes(self, max_cases_per_cta: int = 32):
-        """Build the schedules of every CTA shape a launch may take (512 / 1,024 threads, up to
-        ``max_cases_per_cta`` slots) now rather than on a later launch's critical path."""
+        """Build the schedules of every CTA shape a launch may take by the batch-size and group rules
+        (up to ``max_cases_per_cta`` slots) now rather than on a later launch's critical path."""
         _lib.check(_lib.load().gbpf_prepare_shapes(self._h, int(max_cases_per_cta)), "gbpf_prepare_shapes")
 
     def set_shape(self, units: int, threads_per_cta: int, cases_per_cta: int):
