@@ -287,7 +287,8 @@ int gbpf_group_solve(gbpf_group* g, int njobs, const gbpf_job* jobs, const gbpf_
 /* Device arrays (every pointer of every job on the device). */
 int gbpf_group_solve_device(gbpf_group* g, int njobs, const gbpf_job* jobs, const gbpf_params* p);
 /* Launch shape of later group launches: threads per CTA (0: by the batch-size rule) and the
- * budget of variable buses x case slots a CTA holds per job (0: 16,384). */
+ * budget of variable buses x case slots a CTA holds per job (0: 16,384, and a launch's only job
+ * by the batch-size rule, or within this budget where device memory does not hold its slots). */
 int gbpf_group_set_shape(gbpf_group* g, int threads_per_cta, int slot_budget);
 /* Counters of the last group launch (summed over its jobs). */
 int gbpf_group_stats(gbpf_group* g, gbpf_stats* out);
@@ -435,10 +436,10 @@ int gbpf_branch_flows_device(int nbr, int L, const int32_t* f, const int32_t* t,
                              double* i_max, double* loading, void* stream);
 
 /* Host-only view of the shape rules (runs without a GPU, for tests): the batch rule's CTA shape for
- * `units` cases of a grid on n_sm SMs, and the (threads, slots) pairs that gbpf_prepare_shapes
- * builds there (returns their number, shapes: 2 x max_shapes). No reference counterpart. */
-int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int outages, int* threads_per_cta,
-                        int* cases_per_cta);
+ * `units` cases of a grid on n_sm SMs (slot_budget 0), or the group rule's with a budget, and the (threads, slots) pairs that gbpf_prepare_shapes builds there (returns their
+ * number, shapes: 2 x max_shapes). No reference counterpart. */
+int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int outages, int slot_budget,
+                        int* threads_per_cta, int* cases_per_cta);
 int gbpf_selftest_shapes(int n_sm, int n_var_bus, int max_cases_per_cta, int32_t* shapes, int max_shapes);
 /* Host-only check of the planner and the device schedule (runs without a GPU): plan for
  * `workers` workers, Jacobian at (Vm, Va) with injections S (n complex), the schedule

@@ -430,6 +430,28 @@ void choose_shape(const gbpf_solver* s, long long units, bool mixed, int* NT, in
     *G = s->fixed_G ? s->fixed_G : std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / *NT)));
 }
 
+// Shape rule for a launch over several topologies: threads per CTA by the batch-size rule of
+// choose_shape on the total work; case slots per CTA per job: the batch-size rule's count,
+// reduced for large topologies so that a job's CTA holds at most `slot_budget` (16,384)
+// variable buses' worth of cases -- a large grid's cases then get many workers each, and
+// they set the launch's critical path (measured on GB300, 256 grids of 30..19,423 buses x 16
+// scenarios: one slot per CTA for the largest grids halves the launch).
+void group_shape(int nsm, long long units, int* NT, int* Gmax) {
+    const long long share = (units + nsm - 1) / nsm;
+    int per_sm = 1;
+    while (per_sm < share && per_sm < 64) per_sm *= 2;
+    *NT = per_sm <= 4 ? 1024 : 512;
+    *Gmax = std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / *NT)));
+}
+
+int job_slots(int Gmax, int nv, int budget) {
+    int g = 1;
+    while (g * 2 <= Gmax && (long long)(g * 2) * std::max(1, nv) <= budget) g *= 2;
+    return g;
+}
+
+constexpr int DEFAULT_SLOT_BUDGET = 16384;
+
 // (threads, slots) of every CTA that launches of one grid take with up to `most` slots, but for
 // shapes that a caller sets: 512 threads with any number of slots and 1,024 with up to four by the
 // group rule, what batch_shape gives for any batch, and one slot of each of these sizes for a CTA's
@@ -804,29 +826,7 @@ void fill_common(gbpf::Batch& b, const gbpf_solver* s, const gbpf_params& p) {
     b.rcond_min32 = p.pivot_ratio_single * s->plan.rcond0;
 }
 
-// Shape rule for a launch over several topologies: threads per CTA by the batch-size rule of
-// choose_shape on the total work; case slots per CTA per job: the batch-size rule's count,
-// reduced for large topologies so that a job's CTA holds at most `slot_budget` (16,384)
-// variable buses' worth of cases -- a large grid's cases then get many workers each, and
-// they set the launch's critical path (measured on GB300, 256 grids of 30..19,423 buses x 16
-// scenarios: one slot per CTA for the largest grids halves the launch).
-void group_shape(int nsm, long long units, int* NT, int* Gmax) {
-    const long long share = (units + nsm - 1) / nsm;
-    int per_sm = 1;
-    while (per_sm < share && per_sm < 64) per_sm *= 2;
-    *NT = per_sm <= 4 ? 1024 : 512;
-    *Gmax = std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / *NT)));
-}
-
-int job_slots(int Gmax, int nv, int budget) {
-    int g = 1;
-    while (g * 2 <= Gmax && (long long)(g * 2) * std::max(1, nv) <= budget) g *= 2;
-    return g;
-}
-
 }  // namespace
-
-constexpr int DEFAULT_SLOT_BUDGET = 16384;
 
 // A launch context for several topologies at once: its own stream, scratch, control blocks
 // and staging buffers. The topologies (gbpf_solver) keep their plans; a group launch borrows
@@ -839,8 +839,8 @@ struct gbpf_group {
     HStage hstage;  // iterations and flags of gbpf_group_solve
     gbpf_stats last{};
     int fixed_NT = 0;              // threads per CTA (0: by the group rule)
-    int slot_budget = DEFAULT_SLOT_BUDGET;  // variable buses x case slots a CTA may hold per job (measured best on the
-                                   // 256-grid batch: 8,192 +5 %, 32,768 +8 % time)
+    int slot_budget = 0;           // variable buses x case slots a CTA may hold per job (0: DEFAULT_SLOT_BUDGET,
+                                   // measured best on the 256-grid batch: 8,192 +5 %, 32,768 +8 % time)
     ~gbpf_group() {
         for (DBuf* b : {&scr, &bjobs, &bctl, &btab, &bin, &bout, &bisl}) b->release();
         for (cudaEvent_t e : {e0, e1, c0, c1})
@@ -851,8 +851,10 @@ struct gbpf_group {
 
 namespace {
 
-// One launch over `nj` jobs whose inputs and outputs are device pointers.
-int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p, const char* who) {
+// One launch over `nj` jobs whose inputs and outputs are device pointers. batch_rule: a launch's only
+// job may take the batch rule's shape.
+int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p, const char* who,
+              bool batch_rule = true) {
     long long units = 0;
     for (int j = 0; j < nj; ++j) {
         const gbpf_job& J = jobs[j];
@@ -876,8 +878,10 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     int NT = 0, Gmax = 0;
     const bool mixed = p.precision == 1;
     group_shape(g->nsm, units, &NT, &Gmax);
-    int alone = 0;  // slots of a launch's only job, by its own batch rule
-    if (nj == 1 && !g->fixed_NT && !jobs[0].cases_per_cta && g->slot_budget == DEFAULT_SLOT_BUDGET) {
+    // a launch's only job goes by the batch rule, unless its caller set a slot budget
+    const int budget = g->slot_budget ? g->slot_budget : DEFAULT_SLOT_BUDGET;
+    int alone = 0;  // its slots
+    if (batch_rule && nj == 1 && !g->fixed_NT && !jobs[0].cases_per_cta && !g->slot_budget) {
         batch_shape(g->nsm, std::max(1, jobs[0].solver->plan.nv), units, mixed, jobs[0].out_ptr != nullptr, &NT, &alone);
         Gmax = alone;
     }
@@ -901,7 +905,7 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     // a job whose cases all start from one V0 on the base Ybus without pins gets a shared start
     // (its first evaluation and factorization once, start_kernel)
     auto job_slots_of = [&](const gbpf_job& J) {
-        return J.cases_per_cta ? J.cases_per_cta : alone ? alone : job_slots(Gmax, J.solver->plan.nv, g->slot_budget);
+        return J.cases_per_cta ? J.cases_per_cta : alone ? alone : job_slots(Gmax, J.solver->plan.nv, budget);
     };
     long long bus_cases = 0;
     for (int j = 0; j < nj; ++j) bus_cases += (long long)jobs[j].n_cases * jobs[j].solver->n;
@@ -1034,7 +1038,12 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
         hs[k].rcond_min = mixed ? b.rcond_min32 : b.rcond_min64;
     }
     const int grid = grid_size(g->nsm, occ, want, mixed);
-    CK(g->scr.ensure((size_t)grid * cta_bytes));
+    const cudaError_t room = g->scr.ensure((size_t)grid * cta_bytes);
+    if (room == cudaErrorMemoryAllocation && alone) {  // the group rule's CTAs hold fewer slots
+        (void)cudaGetLastError();
+        return group_run(g, nj, jobs, p, who, false);
+    }
+    CK(room);
     const size_t jobs_bytes = up256((size_t)nj * sizeof(gbpf::Job));
     CK(g->bjobs.ensure(jobs_bytes + hs.size() * sizeof(gbpf::StartJob)));
     CK(cudaMemcpyAsync(g->bjobs.p, hj.data(), (size_t)nj * sizeof(gbpf::Job), cudaMemcpyHostToDevice, g->stream));
@@ -1203,11 +1212,16 @@ int gbpf_prepare_shapes(gbpf_solver* s, int max_cases_per_cta) {
     return 0;
 }
 
-int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int outages, int* threads_per_cta,
-                        int* cases_per_cta) {
-    if (n_sm <= 0 || n_var_bus <= 0 || units <= 0 || !threads_per_cta || !cases_per_cta)
+int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int outages, int slot_budget,
+                        int* threads_per_cta, int* cases_per_cta) {
+    if (n_sm <= 0 || n_var_bus <= 0 || units <= 0 || slot_budget < 0 || !threads_per_cta || !cases_per_cta)
         return fail("selftest_shape: invalid argument");
-    batch_shape(n_sm, n_var_bus, units, mixed != 0, outages != 0, threads_per_cta, cases_per_cta);
+    if (slot_budget) {
+        group_shape(n_sm, units, threads_per_cta, cases_per_cta);
+        *cases_per_cta = job_slots(*cases_per_cta, n_var_bus, slot_budget);
+    } else {
+        batch_shape(n_sm, n_var_bus, units, mixed != 0, outages != 0, threads_per_cta, cases_per_cta);
+    }
     return 0;
 }
 
@@ -2022,7 +2036,7 @@ int gbpf_group_set_shape(gbpf_group* g, int threads_per_cta, int slot_budget) {
         return fail("group_set_shape: threads_per_cta must be 0, 256, 512 or 1024");
     if (slot_budget < 0) return fail("group_set_shape: slot_budget must be >= 0");
     g->fixed_NT = threads_per_cta;
-    g->slot_budget = slot_budget ? slot_budget : 16384;
+    g->slot_budget = slot_budget;
     return 0;
 }
 

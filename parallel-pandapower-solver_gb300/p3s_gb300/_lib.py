@@ -142,8 +142,8 @@ SIGNATURES = {
     "gbpf_selftest_math": (C.c_int, [_dp, C.c_int, _dp, _dp, _dp, _dp, _dp, _dp, _dp]),
     "gbpf_host_alloc": (_vp, [C.c_size_t]),
     "gbpf_host_free": (None, [_vp]),
-    "gbpf_selftest_shape": (C.c_int, [C.c_int, C.c_int, C.c_longlong, C.c_int, C.c_int, C.POINTER(C.c_int),
-                                      C.POINTER(C.c_int)]),
+    "gbpf_selftest_shape": (C.c_int, [C.c_int, C.c_int, C.c_longlong, C.c_int, C.c_int, C.c_int,
+                                      C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "gbpf_selftest_shapes": (C.c_int, [C.c_int, C.c_int, C.c_int, _ip, C.c_int]),
     "gbpf_plan_selftest": (C.c_int, [C.c_int, _ip, _ip, _dp, C.c_int, _ip, C.c_int, _ip, C.c_int, C.c_int, _dp, _dp,
                                      _dp, _dp, _ip, C.c_char_p, C.c_int, C.c_double]),

@@ -11,9 +11,9 @@ from p3s_gb300 import _lib
 GRIDS = (1, 13, 64, 65, 117, 250, 251, 399, 400, 600, 601, 1500, 1999, 3500, 4096, 4097, 8192, 16384, 16385, 19999)
 
 
-def _rule(nsm, nv, units, mixed, outages):
+def _rule(nsm, nv, units, mixed, outages, slot_budget=0):
     nt, g = C.c_int(), C.c_int()
-    assert _lib.load().gbpf_selftest_shape(nsm, nv, units, mixed, outages, C.byref(nt), C.byref(g)) == 0
+    assert _lib.load().gbpf_selftest_shape(nsm, nv, units, mixed, outages, slot_budget, C.byref(nt), C.byref(g)) == 0
     return nt.value, g.value
 
 
@@ -40,3 +40,18 @@ def test_every_shape_of_a_launch_is_prepared(nsm):
             prepared = _prepared(nsm, nv, most)
             assert used <= prepared, (nv, most, used - prepared)
             assert max(g for _, g in prepared) <= most
+
+
+@pytest.mark.parametrize("budget", [1, 8192, 16384, 65536])
+def test_group_shapes_keep_within_the_slot_budget(budget):
+    """Variable buses x slots of a CTA stay within a group's budget (one slot at least), and a server's warm-up,
+    which prepares as many slots as the budget allows, has the shape."""
+    for nv in GRIDS:
+        most = 1
+        while most < 32 and 2 * most * nv <= budget:
+            most *= 2
+        prepared = _prepared(152, nv, most)
+        for units in (*range(1, 152 * 70, 97), 1 << 40):
+            nt, g = _rule(152, nv, units, 0, 0, budget)
+            assert g == 1 or nv * g <= budget, (nv, units, nt, g)
+            assert {(nt, g), (nt, 1)} <= prepared, (nv, units, nt, g)
