@@ -63,7 +63,7 @@ typedef struct gbpf_params {
 /* Topology / schedule facts of a solver (for stats, rooflines and tests). */
 typedef struct gbpf_info {
     int n_bus, nnz_ybus, n_var_bus, n_blocks, n_levels, n_back_levels;
-    int cases_per_cta, threads_per_cta, workers;
+    int cases_per_cta, threads_per_cta, workers; /* the shape of a double batch that fills the device */
     long long factor_pairs, forward_pairs, backward_pairs;
     double rcond0;
     double jinv_norm;    /* estimate of |J^-1| (infinity norm) at the flat start */
@@ -124,13 +124,15 @@ int gbpf_get_stats(gbpf_solver* s, gbpf_stats* out);
  * accuracy statement of the mixed path). No reference counterpart. */
 int gbpf_get_mismatch(gbpf_solver* s, double* out, long long n);
 /* CTA shape (threads per CTA, case slots per CTA) the solver launches for a batch of
- * `units` work items (cases, or lanes), and an override per batch-size class
+ * `units` work items (cases, or lanes) in double precision, the default of gbpf_params
+ * (get_shape_of: in the given gbpf_params.precision), and an override per batch-size class
  * (ceil(log2(units))) -- what an autotuner sets after timing candidate shapes. Results do not
  * depend on the shape (every case runs the same arithmetic); only the speed does.
  * threads_per_cta = cases_per_cta = 0 removes the override. No reference counterpart (the
  * reference's lean LU kernel takes a fixed warps-per-block `slots` argument,
  * nr_polar_solver.py:285-300). */
 int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta);
+int gbpf_get_shape_of(gbpf_solver* s, long long units, int precision, int* threads_per_cta, int* cases_per_cta);
 int gbpf_set_shape(gbpf_solver* s, long long units, int threads_per_cta, int cases_per_cta);
 /* Builds, ahead of use, the schedules of every CTA shape a launch of this topology may take
  * with up to max_cases_per_cta slots by the batch-size and group rules, in either precision, so

@@ -1191,7 +1191,7 @@ int gbpf_get_info(gbpf_solver* s, gbpf_info* o) {
     o->n_levels = p.nlev;
     o->n_back_levels = p.nblev;
     int NT = 0, G = 0;  // the shape of a batch that fills the device
-    choose_shape(s, 1LL << 40, true, &NT, &G);
+    choose_shape(s, 1LL << 40, default_params().precision == 1, &NT, &G);
     o->cases_per_cta = G;
     o->threads_per_cta = NT;
     o->workers = NT / G;
@@ -1236,11 +1236,16 @@ int gbpf_selftest_shapes(int n_sm, int n_var_bus, int max_cases_per_cta, int32_t
     return k;
 }
 
-int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta) {
+int gbpf_get_shape_of(gbpf_solver* s, long long units, int precision, int* threads_per_cta, int* cases_per_cta) {
     if (!s || !threads_per_cta || !cases_per_cta) return fail("null argument");
     if (units <= 0) return fail("get_shape: units must be > 0");
-    choose_shape(s, units, true, threads_per_cta, cases_per_cta);
+    if (precision != 0 && precision != 1) return fail("get_shape: precision must be 0 (double) or 1 (mixed)");
+    choose_shape(s, units, precision == 1, threads_per_cta, cases_per_cta);
     return 0;
+}
+
+int gbpf_get_shape(gbpf_solver* s, long long units, int* threads_per_cta, int* cases_per_cta) {
+    return gbpf_get_shape_of(s, units, default_params().precision, threads_per_cta, cases_per_cta);
 }
 
 int gbpf_set_shape(gbpf_solver* s, long long units, int threads_per_cta, int cases_per_cta) {

@@ -170,10 +170,13 @@ class GpuSolver:
             return None
         return out
 
-    def shape(self, units: int):
+    def shape(self, units: int, precision: str = "double"):
         """(threads per CTA, case slots per CTA) launched for a batch of `units` work items."""
+        if precision not in ("double", "mixed"):
+            raise ValueError(f"precision must be 'double' or 'mixed', got {precision!r}")
         nt, g = C.c_int(), C.c_int()
-        _lib.check(_lib.load().gbpf_get_shape(self._h, int(units), C.byref(nt), C.byref(g)), "gbpf_get_shape")
+        _lib.check(_lib.load().gbpf_get_shape_of(self._h, int(units), int(precision == "mixed"), C.byref(nt),
+                                                 C.byref(g)), "gbpf_get_shape_of")
         return nt.value, g.value
 
     def prepare_shapes(self, max_cases_per_cta: int = 32):

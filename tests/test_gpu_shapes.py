@@ -1,5 +1,5 @@
-"""Group launches of a single job on the GPU: the batch rule's CTA shape unless the caller set a slot budget
-or device memory does not hold its slots; the same bits by every route."""
+"""CTA shapes on the GPU: what is told is launched, and group launches of a single job take the batch rule's
+shape unless the caller set a slot budget or device memory does not hold its slots; the same bits by every route."""
 
 import numpy as np
 import pytest
@@ -54,3 +54,17 @@ def test_an_only_job_runs_where_memory_holds_the_group_rules_slots_only():
         torch.cuda.empty_cache()
     assert shape == (512, 16)  # (the most slots that the group rule gives any job)
     assert np.array_equal(got["V"], want["V"]) and np.array_equal(got["iterations"], want["iterations"])
+
+
+@pytest.mark.parametrize("n,cases", [(118, 1), (118, 4000), (490, 96), (490, 6500)])
+def test_the_shape_told_is_the_shape_launched(n, cases):
+    """Batches whose shape differs between the precisions; without a word the precision is the parameters'
+    default, double."""
+    g = make_grid(n, seed=n, max_drop_pu=0.05)
+    S = scenario_injections(g, cases, seed=1)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    told = {precision: s.shape(cases, precision) for precision in ("double", "mixed")}
+    assert told["double"] != told["mixed"] and s.shape(cases) == told["double"]
+    for precision, shape in told.items():
+        s.solve_batch(S, g.V0, GpuSolver.params(precision=precision))
+        assert (s.stats["threads_per_cta"], s.stats["cases_per_cta"]) == shape
