@@ -909,7 +909,7 @@ int group_run(gbpf_group* g, int nj, const gbpf_job* jobs, const gbpf_params& p,
     };
     long long bus_cases = 0;
     for (int j = 0; j < nj; ++j) bus_cases += (long long)jobs[j].n_cases * jobs[j].solver->n;
-    const bool starts = p.shared_start == 1 || (p.shared_start == 2 && start_pays(g->nsm, units, bus_cases, mixed));
+    const bool starts = p.shared_start && (p.shared_start != 2 || start_pays(g->nsm, units, bus_cases, mixed));
     auto shares = [&](const gbpf_job& J) {
         return starts && J.n_cases >= SHARE_MIN_CASES && !J.v0_per_col && !J.st_ptr && !J.out_ptr && !J.pin &&
                (!mixed || p.vote_rule == 1);

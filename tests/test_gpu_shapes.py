@@ -68,3 +68,17 @@ def test_the_shape_told_is_the_shape_launched(n, cases):
     for precision, shape in told.items():
         s.solve_batch(S, g.V0, GpuSolver.params(precision=precision))
         assert (s.stats["threads_per_cta"], s.stats["cases_per_cta"]) == shape
+
+
+@pytest.mark.parametrize("shared_start", [-1, 0, 1, 2, 3])
+def test_a_group_shares_the_start_for_the_values_a_solver_does(shared_start):
+    """Any value but 0 (never) and 2 (where it pays: not for 200 cases of 65 buses) shares the start."""
+    g = make_grid(65, seed=65, max_drop_pu=0.05)
+    S = scenario_injections(g, 200, seed=1)
+    s = GpuSolver(g.Yp, g.Yj, g.Yx, g.pv, g.pq)
+    p = GpuSolver.params()
+    p.shared_start = shared_start
+    grp = GpuGroup()
+    got, want = grp.solve([GroupJob(s, S, g.V0)], p)[0], s.solve_batch(S, g.V0, p)
+    assert grp.stats["first_steps"] == s.stats["first_steps"] == (0 if shared_start in (0, 2) else 200)
+    assert np.array_equal(got["V"], want["V"]) and np.array_equal(got["iterations"], want["iterations"])
