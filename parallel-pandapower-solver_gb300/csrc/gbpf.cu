@@ -406,10 +406,6 @@ void batch_shape(int nsm, int nv, long long units, bool mixed, bool outages, int
                 *G = slots;
             }
         }
-    if (!*NT) {  // (every candidate is above the cap)
-        *NT = 512;
-        *G = std::max(1, per_sm / 2);
-    }
     fit_outages();
 }
 

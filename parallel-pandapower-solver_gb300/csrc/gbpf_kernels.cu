@@ -708,7 +708,7 @@ __device__ __forceinline__ void lane_forward(const DevPlan& P, const LuLane& L, 
                     if (dinv_smem) dinv_smem[tid] = dinv;
                     // a chain segment's copy (TASK_NOSTORE) only recomputes it; the task itself
                     // records the pivots (a00 and det / a00) and stores the inverse apart, at
-                    // block nblk + row (the Jacobian's diagonal stays for the copies)
+                    // block nblk + row (the diagonal block itself stays for the copies in this level)
                     if (!(task.y & 64)) {
                         pv.see(acc.x);
                         if (task.y & 32) pv.see_ratio(det, acc.x);
@@ -824,36 +824,33 @@ __device__ __forceinline__ void lane_backward(const DevPlan& P, const LuLane& L,
 // Levels with four lanes on one task, one per entry of its 2x2 block, on CTAs of at most 2^QUAD_LG
 // slots (and a CTA's last case). A small CTA has few tasks a level in the narrow levels and waits
 // for each one's chain of instructions; four lanes make that chain a quarter as long -- a pair is
-// two dependent multiply-adds instead of eight, which counts above all in double precision,
-// where an instruction holds its sub-core's FP64 pipe for 64 cycles even if one lane works -- and
-// hold a pair in four registers instead of sixteen, so that four pairs are in flight at once. In
-// the wide levels, which are held by the tasks in flight, one lane a task is the better use of a
-// warp. Entries are formed by the operations of the lane form in its order (the inverse and the
-// scaling exchange entries by shuffles), so results are the same bit for bit. A forward or
-// backward row uses its two row lanes (their neighbours repeat them). The quad programs hold
-// 8 / G tasks a step, their records the first four pairs. Double, factorization and forward
-// substitution of one case over a solve: 118 buses 0.28 -> 0.19 ms, 2,000 buses 0.87 -> 0.68; 744
-// cases of 490 buses (4 slots) 0.86 -> 0.68.
-template <typename real>
+// two dependent multiply-adds instead of eight, and a double-precision instruction holds its
+// sub-core's FP64 pipe for 64 cycles even if one lane works -- and hold a pair in eight registers
+// instead of sixteen, so that two pairs are in flight at once. In the wide levels, which are held
+// by the tasks in flight, one lane a task is the better use of a warp. Entries are formed by the
+// operations of the lane form in its order (the inverse and the scaling exchange entries by
+// shuffles), so results are the same bit for bit. A forward or backward row uses its two row lanes
+// (their neighbours repeat them). The quad programs hold 8 / G tasks a step, their records the
+// first four pairs. Double, factorization and forward substitution of one case over a solve: 118
+// buses 0.28 -> 0.19 ms, 2,000 buses 0.87 -> 0.68; 744 cases of 490 buses (4 slots) 0.86 -> 0.68.
 struct Quad {
-    using B2 = typename V4<real>::t2;
     const DevPlan& P;
     const LuLane& L;
-    real *fa, *fb, *y;        // the slot's first block from (r, 0) and (0, c) on, its first pair
+    double *fa, *fb, *y;      // the slot's first block from (r, 0) and (0, c) on, its first pair
     unsigned step;            // bytes from block to block
     int r, c, wi, lgt;        // this lane's entry of the block; the task of the step, tasks a step (log2)
     unsigned col, rowx, quad; // lanes of the other column / row; the task's four lanes
     int t = 0, t1 = 0;
     int4 next, n01, n23;
-    __device__ __forceinline__ Quad(const DevPlan& P, const LuLane& L, typename V4<real>::t* f, B2* y2)
-        : P(P), L(L), y(reinterpret_cast<real*>(y2 + L.s)), step((unsigned)(4 * sizeof(real)) << L.lg) {
+    __device__ __forceinline__ Quad(const DevPlan& P, const LuLane& L, double4_32a* f, double2* y2)
+        : P(P), L(L), y(reinterpret_cast<double*>(y2 + L.s)), step((unsigned)sizeof(double4_32a) << L.lg) {
         const int lane = threadIdx.x & 31;
         r = (lane >> (L.ll + 1)) & 1;
         c = (lane >> L.ll) & 1;
         wi = lane >> (L.ll + 2);
         lgt = 3 - L.ll;
-        fa = reinterpret_cast<real*>(f + L.s) + 2 * r;
-        fb = reinterpret_cast<real*>(f + L.s) + c;
+        fa = reinterpret_cast<double*>(f + L.s) + 2 * r;
+        fb = reinterpret_cast<double*>(f + L.s) + c;
         col = 1u << L.ll;
         rowx = 2u << L.ll;
         quad = (1u | 1u << col | 1u << rowx | 1u << (col | rowx)) << (lane & ~(int)(col | rowx));
@@ -865,33 +862,33 @@ struct Quad {
         n23 = __ldg(rec + 2);
     }
     // row r of a block, entry (0, c) of a block, component r of a row's pair
-    __device__ __forceinline__ B2& row_of(int x) const {
-        return *(B2*)((char*)fa + (unsigned long long)(unsigned)x * step);
+    __device__ __forceinline__ double2& row_of(int x) const {
+        return *(double2*)((char*)fa + (unsigned long long)(unsigned)x * step);
     }
-    __device__ __forceinline__ real* col_of(int x) const {
-        return (real*)((char*)fb + (unsigned long long)(unsigned)x * step);
+    __device__ __forceinline__ double* col_of(int x) const {
+        return (double*)((char*)fb + (unsigned long long)(unsigned)x * step);
     }
-    __device__ __forceinline__ real& entry(int x) const { return reinterpret_cast<real*>(&row_of(x))[c]; }
-    __device__ __forceinline__ B2& pair(int x) const {
-        return *(B2*)((char*)y + (unsigned long long)(unsigned)x * (step / 2));
+    __device__ __forceinline__ double& entry(int x) const { return reinterpret_cast<double*>(&row_of(x))[c]; }
+    __device__ __forceinline__ double2& pair(int x) const {
+        return *(double2*)((char*)y + (unsigned long long)(unsigned)x * (step / 2));
     }
-    __device__ __forceinline__ real& comp(int x) const { return reinterpret_cast<real*>(&pair(x))[r]; }
+    __device__ __forceinline__ double& comp(int x) const { return reinterpret_cast<double*>(&pair(x))[r]; }
     // acc -= (row r of block x) . (b0, b1): for factor tasks column c of block y, for
     // substitution rows the pair (y0, y1) of row y
-    __device__ __forceinline__ real sum(real acc, int4 task, int4 q01, int4 q23, bool subst) const {
+    __device__ __forceinline__ double sum(double acc, int4 task, int4 q01, int4 q23, bool subst) const {
         auto a_of = [&](int x) { return row_of(x); };
         auto b_of = [&](int yb) {
-            B2 b;
+            double2 b;
             if (subst) {
                 b = pair(yb);
             } else {
-                const real* p = col_of(yb);
+                const double* p = col_of(yb);
                 b.x = p[0];
                 b.y = p[2];
             }
             return b;
         };
-        auto sub = [&](const B2& a, const B2& b) { acc = fmadd(-a.y, b.y, fmadd(-a.x, b.x, acc)); };
+        auto sub = [&](const double2& a, const double2& b) { acc = fmadd(-a.y, b.y, fmadd(-a.x, b.x, acc)); };
         for (int p = task.z; p < task.w; p += 4) {
             const int m = task.w - p;
             if (p > task.z) {
@@ -900,17 +897,14 @@ struct Quad {
                 q01 = make_int4(i0.x, i0.y, i1.x, i1.y);
                 q23 = make_int4(i2.x, i2.y, i3.x, i3.y);
             }
-            // (float: all four in flight; double: two and two, in as many registers)
-            constexpr bool ALL = sizeof(real) == 4;
-            B2 a0 = a_of(q01.x), b0 = b_of(q01.y), a1 = {}, b1 = {}, a2 = {}, b2 = {}, a3 = {}, b3 = {};
+            // (two and two: four in flight would take twice the registers)
+            double2 a0 = a_of(q01.x), b0 = b_of(q01.y), a1 = {}, b1 = {}, a2 = {}, b2 = {}, a3 = {}, b3 = {};
             if (m > 1) {
                 a1 = a_of(q01.z);
                 b1 = b_of(q01.w);
             }
-            if (!ALL) {
-                sub(a0, b0);
-                if (m > 1) sub(a1, b1);
-            }
+            sub(a0, b0);
+            if (m > 1) sub(a1, b1);
             if (m > 2) {
                 a2 = a_of(q23.x);
                 b2 = b_of(q23.y);
@@ -919,21 +913,17 @@ struct Quad {
                 a3 = a_of(q23.z);
                 b3 = b_of(q23.w);
             }
-            if (ALL) {
-                sub(a0, b0);
-                if (m > 1) sub(a1, b1);
-            }
             if (m > 2) sub(a2, b2);
             if (m > 3) sub(a3, b3);
         }
         return acc;
     }
 
-    __device__ __forceinline__ void forward(const double2* R2, Pivots<real>& pv, int h0, int h1) {
+    __device__ __forceinline__ void forward(const double2* R2, Pivots<double>& pv, int h0, int h1) {
         const double* const R = reinterpret_cast<const double*>(R2);
         const int warp = threadIdx.x >> 5;
         const bool act = L.act, factor = L.factor;
-        real dinv = 0;  // this lane's entry of the last inverse diagonal block
+        double dinv = 0.0;  // this lane's entry of the last inverse diagonal block
         if (act) {
             const int* ptr = P.qptrA + warp * (P.nlev + 1) + h0;
             t = __ldg(ptr);
@@ -949,27 +939,25 @@ struct Quad {
                     fetch(P.qtaskA);
                     const int kind = task.y & 3;
                     if (task.x < 0 || (kind != 3 && !factor)) continue;
-                    real acc;
+                    double acc;
                     if (kind == 3) {
                         if (task.y & 128)  // its leading pairs are already summed (TASK_CONT)
                             acc = comp(task.x);
-                        else if constexpr (sizeof(real) == 4)
-                            acc = d2f_fast(R[2 * (((size_t)task.x << L.lg) + L.s) + r]);
                         else
                             acc = R[2 * (((size_t)task.x << L.lg) + L.s) + r];
                     } else {
-                        acc = (task.y & 16) ? (real)0 : entry(task.x);
+                        acc = (task.y & 16) ? 0.0 : entry(task.x);
                     }
                     acc = sum(acc, task, q01, q23, kind == 3);
                     if (kind == 3) {
                         if (c == 0) comp(task.x) = acc;
                     } else if (kind == 0) {  // (entries x y z w of the block; this lane's is acc)
-                        const real v1 = __shfl_xor_sync(quad, acc, col), v2 = __shfl_xor_sync(quad, acc, rowx);
-                        const real v3 = __shfl_xor_sync(quad, acc, col | rowx);
+                        const double v1 = __shfl_xor_sync(quad, acc, col), v2 = __shfl_xor_sync(quad, acc, rowx);
+                        const double v3 = __shfl_xor_sync(quad, acc, col | rowx);
                         const bool on_diag = r == c;  // lane of x or w: (acc, v3) = (x, w), (v1, v2) = (y, z); else crosswise
-                        const real det = fmadd(on_diag ? acc : v1, on_diag ? v3 : v2,
-                                               -mulr(on_diag ? v1 : acc, on_diag ? v2 : v3));
-                        const real inv = (real)1 / det;
+                        const double det = fmadd(on_diag ? acc : v1, on_diag ? v3 : v2,
+                                                 -mulr(on_diag ? v1 : acc, on_diag ? v2 : v3));
+                        const double inv = 1.0 / det;
                         dinv = (on_diag ? v3 : -acc) * inv;
                         if (!(task.y & 64)) {
                             if (r + c == 0) {
@@ -979,7 +967,7 @@ struct Quad {
                             entry(P.nblk + (task.y >> 8)) = dinv;
                         }
                     } else if (task.y & 8) {
-                        const real va = __shfl_xor_sync(quad, acc, col), vd = __shfl_xor_sync(quad, dinv, rowx);
+                        const double va = __shfl_xor_sync(quad, acc, col), vd = __shfl_xor_sync(quad, dinv, rowx);
                         entry(task.x) =
                             fmadd(c ? va : acc, r ? vd : dinv, mulr(c ? acc : va, r ? dinv : vd));
                     } else {
@@ -1009,10 +997,10 @@ struct Quad {
                     ++t;
                     fetch(P.qtaskC);
                     if (task.x < 0) continue;
-                    const B2 d = row_of(task.y);
-                    const real acc = sum(comp(task.x), task, q01, q23, true);
-                    const real other = __shfl_xor_sync(quad, acc, rowx);
-                    const real o = fmadd(d.x, r ? other : acc, mulr(d.y, r ? acc : other));
+                    const double2 d = row_of(task.y);
+                    const double acc = sum(comp(task.x), task, q01, q23, true);
+                    const double other = __shfl_xor_sync(quad, acc, rowx);
+                    const double o = fmadd(d.x, r ? other : acc, mulr(d.y, r ? acc : other));
                     if (c == 0) comp(task.x) = o;
                 }
                 t1 = t2;
@@ -1048,9 +1036,9 @@ __device__ void lu_pass(const DevPlan& P, typename V4<real>::t* fac, const doubl
     if constexpr (sizeof(real) == 8 && QUADS) {
         const int hq = factor_any ? P.quad_from : P.nlev;
         lane_forward<real>(P, L, fac, R, y, dinv_smem, pv, 0, hq);
-        if (hq < P.nlev) Quad<real>(P, L, fac, y).forward(R, pv, hq, P.nlev);
+        if (hq < P.nlev) Quad(P, L, fac, y).forward(R, pv, hq, P.nlev);
         if constexpr (TIMED) phase_mark(ph, clk, 1);
-        if (BACK && P.quad_to) Quad<real>(P, L, fac, y).backward(0, P.quad_to);
+        if (BACK && P.quad_to) Quad(P, L, fac, y).backward(0, P.quad_to);
         if (BACK) lane_backward<real>(P, L, fac, y, P.quad_to, P.nblev);
     } else {
         lane_forward<real>(P, L, fac, R, y, dinv_smem, pv, 0, P.nlev);
@@ -1186,7 +1174,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
     // factors; s_nofac: this step solves with factors it does not compute (chord or first)
     __shared__ int s_first[MAX_SLOTS], s_nofac[MAX_SLOTS];
     // slots with a point to form and evaluate in this pass, and whether the per-bus phases deal
-    // their threads to those slots only (see `lanes_of`)
+    // their threads to those slots only (see `deal`)
     __shared__ int s_act[MAX_SLOTS], s_nact;
     __shared__ int s_share;  // the launch's shared start is usable (its factorization passed)
     // outage stamps of every slot (entry values, then rows), only in launches that have any
