@@ -166,8 +166,9 @@ __global__ void __launch_bounds__(NT) islands_kernel(int n, int m, const int* f,
 // makes those reads 292 cycles each in L2, over several passes with five block barriers each.
 // Measured, 2,000 buses: 3,000 cases 0.43 ms there, 0.17 here; 200 cases 75 and 59 us, one case 70
 // and 45 us (118 buses 15 and 9, 3,500 buses 107 and 81 us; 3,500 x 3,000 cases 0.76 and 0.40 ms).
-// A CTA takes no more threads, registers or shared memory than a 512-thread CTA of the Newton kernel:
-// wherever that fits beside a resident stream launch, so does this.
+// A CTA takes no more threads, registers or shared memory (up to 40 KB) than a 512-thread CTA of a
+// stream launch: wherever one of those fits beside a resident one, so does this. (A mixed Newton CTA of
+// another launch takes 6 KB without outage stamps.)
 constexpr int TPC = 128;              // threads per case
 constexpr int MAX_PER_THREAD = 32;    // buses of a thread, by the bits of a word
 constexpr int MAX_SHARED_BUS = MAX_PER_THREAD * TPC;

@@ -119,7 +119,8 @@ std::vector<int> rcm_order(int n, const int* Yp, const int* Yj) {
 // one worker; a chain heavier than its level's share of a worker (total weight / workers) is cut
 // into segments of at most that share (at least one L block each), every segment after the first
 // led by a copy of the diagonal task flagged TASK_NOSTORE (it recomputes the inverse from the
-// Jacobian's diagonal, which the pass leaves in place).
+// diagonal block, which no task of its level writes; cut_long may have added leading pairs to it in
+// a lower one).
 //
 // A warp's workers run in step, so a level's units (chains, segments, single tasks) are first
 // tied into bundles of wpw units alike -- factor and forward units apart, neighbours in weight --

@@ -15,15 +15,16 @@
 //  * Factor entries are computed in Crout form, one task per block; a pivot's diagonal block
 //    and its column of L form one chain on one worker (the inverse diagonal stays in
 //    registers and scales each L block as it is computed: no separate scaling pass, one
-//    barrier per level). The inverse diagonal is stored apart, at block nblk + row, so the
-//    Jacobian's diagonal block stays intact through the pass: a chain heavier than its
-//    level's share of a worker is cut into segments, each later segment led by a copy of
-//    the diagonal task that recomputes the inverse from it without storing anything. Tasks
-//    and chain segments are grouped by elimination-tree height (level), bundled with others of
-//    like length into steps of a warp, and the bundles dealt to the CTA's warps longest-first
-//    onto the least-loaded one (Schedule below). Pairs of a long task whose operands are final
-//    earlier are summed in an earlier level. The forward substitution rides along in the same
-//    levels.
+//    barrier per level). The inverse diagonal is stored apart, at block nblk + row, and no task
+//    writes a diagonal block in its own level: a chain heavier than its level's share of a
+//    worker is cut into segments, each later segment led by a copy of the diagonal task that
+//    recomputes the inverse from it without storing anything. Tasks and chain segments are
+//    grouped by elimination-tree height (level), bundled with others of like length into steps
+//    of a warp, and the bundles dealt to the CTA's warps longest-first onto the least-loaded one
+//    (Schedule below). Pairs of a long task whose operands are final earlier are summed in an
+//    earlier level, also into a diagonal block: after a pass it may hold a part of its sum, so
+//    that every factorization needs a Jacobian evaluated anew. The forward substitution rides
+//    along in the same levels.
 #pragma once
 
 #include <cstdint>
