@@ -888,8 +888,9 @@ extern "C" int gbpf_plan_selftest(int n, const int32_t* Yp, const int32_t* Yj, c
                                   const double* Vm, const double* Va, const double* S, double* dx, int32_t* shape,
                                   char* msg, int msglen, double chain_cap) {
     gbpf::Plan p;
-    std::string e = chain_cap >= 0.0 ? gbpf::build_plan(p, n, Yp, Yj, nnz, pv, npv, pq, npq, workers, chain_cap)
-                                     : std::string("chain_cap must be >= 0");
+    std::string e = chain_cap >= 0.0
+                        ? gbpf::build_plan(p, n, Yp, Yj, nnz, pv, npv, pq, npq, std::max(1, workers), chain_cap)
+                        : std::string("chain_cap must be >= 0");
     if (e.empty()) {
         std::vector<double> blk(4 * ((size_t)p.nblk + p.nv)), R(2 * (size_t)std::max(p.nv, 1)),
             y(2 * (size_t)std::max(p.nv, 1));

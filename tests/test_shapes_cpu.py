@@ -1,5 +1,5 @@
 """The CTA shape rules without a GPU: batches of every size up to where the rule is constant, small to
-very large grids, both precisions, with and without outages."""
+very large grids, both precisions, with and without outages; and the edges of the plan check's arguments."""
 
 import ctypes as C
 
@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 
 from p3s_gb300 import _lib
+from p3s_gb300.synthetic import make_grid
+from test_host_cpu import _selftest
 
 GRIDS = (1, 13, 64, 65, 117, 250, 251, 399, 400, 600, 601, 1500, 1999, 3500, 4096, 4097, 8192, 16384, 16385, 19999)
 
@@ -55,3 +57,9 @@ def test_group_shapes_keep_within_the_slot_budget(budget):
             nt, g = _rule(152, nv, units, 0, 0, budget)
             assert g == 1 or nv * g <= budget, (nv, units, nt, g)
             assert {(nt, g), (nt, 1)} <= prepared, (nv, units, nt, g)
+
+
+@pytest.mark.parametrize("workers", [0, -3])
+def test_a_plan_for_no_workers_is_checked_with_one(workers):
+    err, _ = _selftest(make_grid(30, seed=4), workers)
+    assert err < 1e-9, err  # the bound of the other plan checks
