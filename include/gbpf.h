@@ -445,7 +445,8 @@ int gbpf_selftest_shape(int n_sm, int n_var_bus, long long units, int mixed, int
 int gbpf_selftest_shapes(int n_sm, int n_var_bus, int max_cases_per_cta, int32_t* shapes, int max_shapes);
 /* Host-only check of the planner and the device schedule (runs without a GPU): plan for
  * `workers` workers, Jacobian at (Vm, Va) with injections S (n complex), the schedule
- * executed serially with a structural race check per level. dx (n x 2): Newton step per
+ * executed serially with a structural race check per level (with a multiple of 64 workers also
+ * the one for four lanes a task, whose step must have the same bits). dx (n x 2): Newton step per
  * bus (angle, magnitude). shape (7): n_var_bus, n_blocks, levels, back levels, factor /
  * forward / backward pairs. No reference counterpart: the reference's numpy plan executor
  * (lean_lu_plan.py:324-360) plays this role for its own plan. */

@@ -895,7 +895,22 @@ extern "C" int gbpf_plan_selftest(int n, const int32_t* Yp, const int32_t* Yj, c
         std::vector<double> blk(4 * ((size_t)p.nblk + p.nv)), R(2 * (size_t)std::max(p.nv, 1)),
             y(2 * (size_t)std::max(p.nv, 1));
         gbpf::host_eval(p, Yp, Yj, Yx, Vm, Va, S, nullptr, blk.data(), R.data());
+        const std::vector<double> jac = blk;
         e = gbpf::schedule_selftest(p, blk.data(), R.data(), y.data());
+        if (e.empty() && p.warp % 4 == 0) {  // the same tasks as dealt for four lanes each: the same bits
+            gbpf::Schedule lanes, quad;
+            gbpf::make_schedule(p, p.W / p.warp, p.warp, lanes, chain_cap, &quad);
+            gbpf::Plan q = p;
+            q.W = quad.nwarps * quad.wpw;
+            q.warp = quad.wpw;
+            q.taskA = quad.taskA, q.ptrA = quad.ptrA;
+            q.taskF = quad.taskF, q.ptrF = quad.ptrF;
+            q.taskC = quad.taskC, q.ptrC = quad.ptrC;
+            std::vector<double> blk4 = jac, y4(y.size());
+            e = gbpf::schedule_selftest(q, blk4.data(), R.data(), y4.data());
+            if (e.empty() && std::memcmp(y4.data(), y.data(), y.size() * sizeof(double))) e = "another step";
+            if (!e.empty()) e = "quads: " + e;
+        }
         if (e.empty()) {
             for (int b = 0; b < n; ++b) {
                 const int r = p.row_of_bus[b];
