@@ -426,9 +426,9 @@ void choose_shape(const gbpf_solver* s, long long units, bool mixed, int* NT, in
     *G = s->fixed_G ? s->fixed_G : std::min(gbpf::MAX_SLOTS, std::max(1, per_sm / (1024 / *NT)));
 }
 
-// Shape rule for a launch over several topologies: threads per CTA by the batch-size rule of
-// choose_shape on the total work; case slots per CTA per job: the batch-size rule's count,
-// reduced for large topologies so that a job's CTA holds at most `slot_budget` (16,384)
+// Shape rule for a launch over several topologies: the total's share of an SM rounded up to a power of
+// two, up to four slots on one CTA of 1,024 threads, more on two of 512; case slots per CTA per job:
+// that count, reduced for large topologies so that a job's CTA holds at most `slot_budget` (16,384)
 // variable buses' worth of cases -- a large grid's cases then get many workers each, and
 // they set the launch's critical path (measured on GB300, 256 grids of 30..19,423 buses x 16
 // scenarios: one slot per CTA for the largest grids halves the launch).

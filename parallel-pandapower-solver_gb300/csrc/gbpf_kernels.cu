@@ -1579,7 +1579,7 @@ __global__ void __launch_bounds__(NTB, 1024 / NTB) newton_kernel(const Launch L)
         // slots, 10 busy: evaluation 1.93 ms mixed, 2.09 dealt; N-1 sweeps equal either way). One busy
         // slot alone has all threads on any CTA: with its share of a full CTA, 16 of 512, an hour without
         // a solution added 13.3 ms to a double series of 8,760 hours of 2,000 buses, and adds 2.4 (mixed
-        // 11.0 and 4.3).
+        // 11.0 and 3 to 4).
         auto dealt = [&]() { return s_nact <= 1 || (4 * s_nact <= 3 * G && G < 16); };
         auto deal = [&](int& slot, int& first, int& stride) {
             if (dealt()) {

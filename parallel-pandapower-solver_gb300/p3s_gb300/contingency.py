@@ -173,7 +173,7 @@ def solve_contingencies(grid, reslack_islands: bool = False, tol: float = 1e-8, 
     solve's launch (no per-case arrays cross the bus but the results). Unserved buses come back
     as NaN; ``served`` is the launch's own islanding mask. ``return_islands`` adds the island
     labels and reference buses (one more islanding call). ``cases_per_cta`` /
-    ``threads_per_cta``: the launch's CTA shape (0: the group rule), e.g. from a tuner."""
+    ``threads_per_cta``: the launch's CTA shape (0: the batch rule's for outages), e.g. from a tuner."""
     from .group import GpuGroup, GroupJob
 
     n = grid.n
